@@ -127,7 +127,7 @@ extern "C" axon_status axon_load(axon_net* net, const char* path, axon_ckpt_meta
   st = net->write(AXON_BUF_THETA, zeros.data(), 16);
   if (st != AXON_OK) return st;
   net->initialized = true;
-  net->w3b_valid = false;
+  net->w3b_valid = net->w3p_valid = false;
   if (meta) *meta = m;
   return AXON_OK;
 }

@@ -155,6 +155,8 @@ void axon_net::release() {
   io.release();
   if (w3b) cudaFree(w3b);
   w3b = nullptr;
+  if (w3p) cudaFree(w3p);
+  w3p = nullptr;
   if (base) cudaFree(base);
   if (hstim) cudaFreeHost(hstim);
   if (hscratch) cudaFreeHost(hscratch);
@@ -173,7 +175,7 @@ axon_status axon_net::init(uint32_t seed) {
   CK(cudaMemsetAsync(d.stats, 0, 1024 * 4, stream));
   CK(cudaStreamSynchronize(stream));
   initialized = true;
-  w3b_valid = false;
+  w3b_valid = w3p_valid = false;
   return AXON_OK;
 }
 
@@ -206,7 +208,7 @@ axon_status axon_net::present(const uint32_t* stim, uint32_t T, uint32_t clampSt
   PresentCfg pc = present_cfg(T, clampSteps, learn, useBias);
   pc.missing = inject_missing;
   inject_missing = 0;
-  if (learn) w3b_valid = false;
+  if (learn) w3b_valid = w3p_valid = false;
   CK(cudaEventRecord(ev0, stream));
   CK(launch_present(d, pc, shape, stream));
   CK(cudaEventRecord(ev1, stream));
@@ -276,7 +278,7 @@ axon_status axon_net::write(axon_buf which, const uint32_t* host, uint64_t words
   CK(cudaMemcpyAsync(p, host, words * 4, cudaMemcpyHostToDevice, stream));
   CK(cudaStreamSynchronize(stream));
   if (which == AXON_BUF_W0 || which == AXON_BUF_CONN) initialized = true;
-  if (which == AXON_BUF_W3) w3b_valid = false;
+  if (which == AXON_BUF_W3) w3b_valid = w3p_valid = false;
   return AXON_OK;
 }
 
@@ -363,7 +365,7 @@ axon_status axon_net::profile_present(const uint32_t* stim, uint32_t T, uint32_t
   NetDev dd = d;
   dd.prof = (unsigned long long*)tmp.p;
   const PresentCfg pc = present_cfg(T, clampSteps, learn, useBias);
-  if (learn) w3b_valid = false;
+  if (learn) w3b_valid = w3p_valid = false;
   CK(cudaEventRecord(ev0, stream));
   CK(launch_present(dd, pc, shape, stream));
   CK(cudaEventRecord(ev1, stream));
@@ -394,6 +396,6 @@ axon_status axon_net::clone_from(const axon_net& src) {
   CK(cudaMemcpyAsync(base, src.base, base_bytes, cudaMemcpyDeviceToDevice, stream));
   CK(cudaStreamSynchronize(stream));
   initialized = true;
-  w3b_valid = false;
+  w3b_valid = w3p_valid = false;
   return AXON_OK;
 }

@@ -10,6 +10,7 @@
 
 #include "../../include/axon_capi.h"
 #include "batch.cuh"
+#include "planes.cuh"
 #include "plain.cuh"
 
 namespace axon {
@@ -82,6 +83,11 @@ struct axon_net {
   axon_status recall(const uint32_t* cues, uint32_t B, const axon_recall_args& a, const uint32_t* refBall,
                      uint32_t* finalOut, uint32_t* hist, uint32_t* stats, uint32_t* driveLog, bool dev, double* ms);
   axon_status ensure_w3b();
+  uint32_t* w3p = nullptr;      // W3 in the bit-plane layout (planes.cuh), rebuilt when weights change
+  bool w3p_valid = false;
+  axon_status ensure_w3p();
+  axon_status recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
+                            uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog);
   // the batched readout as a captured CUDA graph, with the arguments it was captured for
   cudaGraphExec_t recallGraph = nullptr;
   std::vector<uint64_t> recallKey;

@@ -582,7 +582,7 @@ axon_status MultiRun::run(const uint32_t* seeds, const uint32_t* nstim, axon_mul
   }
   R.gpu_ms = ms;
   for (uint32_t i = 0; i < n_; ++i) {
-    nets_[i]->w3b_valid = false;
+    nets_[i]->w3b_valid = nets_[i]->w3p_valid = false;
     R.steps += plans_[i].steps;
     R.train_steps += plans_[i].trainSteps;
   }

@@ -1,0 +1,73 @@
+// Host/device interface of the bit-plane batched readout (planes.cu).
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace axon {
+
+// Transposed W3 ("W3P"): per (column, branch, word of the presynaptic group) a block of
+// kPlaneBlk words: 32 masks, mask j = the postsynaptic neurons (bit = lane) whose synapse
+// with presynaptic neuron j is functional; then the six bit planes of the row counts (plane
+// i = the neurons whose number of functional synapses in the word has bit i set); then two
+// zero words, which padding entries of a record's position list point at.
+constexpr uint32_t kPlaneBlk = 40;
+constexpr uint32_t kPlaneTile = 8u * kPlaneBlk;     // one (column, branch)
+constexpr uint32_t kPlaneCol = 32u * kPlaneTile;    // one column
+constexpr uint32_t kPlanes = 14;                    // bit planes of a per-neuron drive (below 2^14)
+constexpr uint32_t kPlanesMaxB = 512;               // trajectories per launch (the host splits larger batches)
+constexpr uint32_t kPlanesVals = 1536;              // candidates a phase-2 group keeps in shared memory
+constexpr uint32_t kPlanesList = 512;               // gated columns it lists there
+constexpr uint32_t kPlanesThreads = 640;  // 96 registers: no spills in phase 1
+
+struct PlanesDev {
+  const uint32_t* W3P;      // [ncol][kPlaneCol]
+  const uint32_t* conn;     // [ncol*32]
+  const uint32_t* biasP;    // [ncol][16] planes of min(bias >> shift, 2^14 - 1), or null (no bias)
+  const uint32_t* multM;    // [ncol] neurons with multiplicity > 1 (with refBall)
+  const uint32_t* stims;    // [B][ncol] clamp patterns
+  const uint32_t* refBall;  // [B][ncol] logged reference assemblies, or null
+  uint32_t* act;            // [2][ngrp][nblk] by step parity: bit j of word (g, k) = trajectory 32k + j spikes in group g
+  uint4* rec;               // [B][ngrp + ncol] per group the record of its first nonzero spike word, then per
+                            // column the records of the further ones
+  uint32_t* drv;            // [ncol][32 * nblk] column drives of the step
+  uint32_t* candB;          // [B][ncol/32] candidates of the step, a bit per column (zeroed before the launch)
+  uint4* candP;             // [B][ncol][4] their drive planes (words 0..13) and column drives (word 14)
+  uint32_t* ball;           // [B][ncol] ballots of a step with more than kPlanesList gated columns
+  uint32_t* thPrev;         // [2][B] the last two thresholds, by step parity
+  uint32_t* finalOut;       // [B][ncol] spikes of the last step (zeroed before the launch), or null
+  uint32_t* hist;           // [B][T][ncol] spikes of every step (zeroed before the launch), or null
+  uint32_t* stats;          // [B][1024] counters (zeroed before the launch), or null
+  uint32_t* driveLog;       // [B][256] member-drive log (accumulated), or null
+  uint32_t* bar;            // grid barrier counter
+  uint32_t* err;            // device error word
+};
+
+struct PlanesCfg {
+  uint32_t ncol, incols, B, T, clampSteps, k, dthr, mode, targetCols, topkPar;
+  uint32_t bst;          // dendritic bonus per branch at or above dthr: boost (mode 1), 0 (mode 0)
+  uint32_t slabFull;     // 1: every column with a positive drive is a candidate
+  uint32_t slabAlways;   // 1: the first step after the clamp takes no floor of its own
+  uint32_t ns, nl, ng;   // tile slots, list slots (0 when direct), phase-2 groups
+  uint32_t nsl, nll;     // log2 of ns and nl
+  uint32_t ls;           // log2 of the lanes per trajectory in phase 1
+  uint64_t waitNs;
+};
+
+struct PlanesShape {
+  int grid;
+  uint32_t direct;  // 1: tiles read through L2 as needed (few trajectories), 0: column tiles staged in shared memory
+  size_t smem;
+};
+
+// Launch shape for B trajectories: fills the last fields of c.
+PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c);
+cudaError_t planes_max_blocks_per_sm(const PlanesCfg& c, const PlanesShape& s, int* out);
+cudaError_t launch_recall_planes(const PlanesDev& d, const PlanesCfg& c, const PlanesShape& s, cudaStream_t st);
+// W3 [col][s][j][lane][comp] -> W3P
+cudaError_t launch_make_w3p(const uint4* W3, uint32_t* W3P, uint32_t ncol, cudaStream_t st);
+// bias planes and multiplicity masks (either output may be null)
+cudaError_t launch_planes_aux(const uint32_t* bias, uint32_t biasShift, const uint32_t* mult, uint32_t* biasP,
+                              uint32_t* multM, uint32_t ncol, cudaStream_t st);
+
+}  // namespace axon

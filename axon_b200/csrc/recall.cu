@@ -47,9 +47,126 @@ axon_status axon_net::ensure_w3b() {
   return AXON_OK;
 }
 
+axon_status axon_net::ensure_w3p() {
+  if (w3p_valid) return AXON_OK;
+  if (!w3p) {
+    if (cudaMalloc(&w3p, (size_t)ncol * kPlaneCol * 4) != cudaSuccess) {
+      cudaGetLastError();
+      w3p = nullptr;
+      return set_error(AXON_ENOMEM, "W3 plane layout allocation failed");
+    }
+  }
+  CK(launch_make_w3p(d.W3, w3p, ncol, stream));
+  w3p_valid = true;
+  return AXON_OK;
+}
+
 namespace {
 size_t al(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 }  // namespace
+
+namespace {
+// The bit-plane kernel takes readouts whose per-neuron drives stay below 2^14 (drive << 13 |
+// column fits one word), without facilitation and on the CUDA cores.
+bool planes_apply(const axon_cfg& cfg, const axon_recall_args& a) {
+  const uint64_t maxAcc = cfg.mode == 2 ? 32ull : 32ull * (256ull + (cfg.mode == 1 ? cfg.boost : 0u));
+  return a.contraction == AXON_CONTRACT_POPC && cfg.facil == 0u && maxAcc < (1ull << kPlanes) && cfg.ncol <= 8192u;
+}
+}  // namespace
+
+axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
+                                    uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog) {
+  const uint32_t ngrp = ncol / 8u, nl = (B + kPlanesMaxB - 1u) / kPlanesMaxB, Bc = (B + nl - 1u) / nl;  // launches, trajectories of one
+  const PresentCfg pc = present_cfg(a.T, a.clamp_steps, false, a.use_bias);
+  PlanesCfg c{};
+  c.ncol = ncol; c.incols = cfg.incols; c.T = a.T; c.clampSteps = a.clamp_steps;
+  c.k = pc.k; c.dthr = pc.dthr; c.mode = pc.mode; c.targetCols = pc.targetCols; c.topkPar = pc.topkPar;
+  c.bst = cfg.mode == 1 ? cfg.boost : 0u;
+  c.slabFull = a.slab == AXON_SLAB_FULL ? 1u : 0u;
+  c.slabAlways = a.slab == AXON_SLAB_FLOOR_ALWAYS ? 1u : 0u;
+  c.waitNs = wait_ns;
+  const size_t nblk = (Bc + 31u) / 32u, bnc = (size_t)Bc * ncol;
+  // zeroed before every launch: activity words of both parities, candidate bits, thresholds,
+  // the barrier word
+  const size_t zBytes = al(2ull * ngrp * nblk * 4) + al((size_t)Bc * (ncol / 32u) * 4) + al((size_t)Bc * 8) + 256;
+  const size_t need = zBytes + al((size_t)Bc * (ngrp + ncol) * 16) + al((size_t)ncol * nblk * 32 * 4) +
+                      al(bnc * 64) + al(bnc * 4) + al((size_t)ncol * 64) + al((size_t)ncol * 4);
+  axon_status st = scratch.ensure(need);
+  if (st != AXON_OK) return st;
+  char* p = (char*)scratch.p;
+  auto take = [&](size_t bytes) { char* r = p; p += al(bytes); return r; };
+  PlanesDev d0{};
+  char* zero = p;
+  d0.act = (uint32_t*)take(2ull * ngrp * nblk * 4);
+  d0.candB = (uint32_t*)take((size_t)Bc * (ncol / 32u) * 4);
+  d0.thPrev = (uint32_t*)take((size_t)Bc * 8);
+  d0.bar = (uint32_t*)take(256);
+  d0.rec = (uint4*)take((size_t)Bc * (ngrp + ncol) * 16);
+  d0.drv = (uint32_t*)take((size_t)ncol * nblk * 32 * 4);
+  d0.candP = (uint4*)take(bnc * 64);
+  d0.ball = (uint32_t*)take(bnc * 4);
+  uint32_t* biasP = (uint32_t*)take((size_t)ncol * 64);
+  uint32_t* multM = (uint32_t*)take((size_t)ncol * 4);
+  d0.W3P = w3p;
+  d0.conn = d.conn;
+  d0.biasP = pc.useBias ? biasP : nullptr;
+  d0.multM = multM;
+  d0.err = d.err;
+  // everything the launches depend on: a captured graph is replayed only for the same key
+  const std::vector<uint64_t> key = {(uint64_t)dCues, (uint64_t)dRef, (uint64_t)dFinal, (uint64_t)dHist,
+                                     (uint64_t)dStats, (uint64_t)dLog, (uint64_t)scratch.p, (uint64_t)w3p, B, a.T,
+                                     a.clamp_steps, a.use_bias, wait_ns, a.contraction, a.slab, 1ull};
+  const bool graph = a.graph != 0u;
+  const bool replay = graph && recallGraph && key == recallKey;
+  if (graph && !replay) {
+    if (recallGraph) cudaGraphExecDestroy(recallGraph);
+    recallGraph = nullptr;
+    recallKey.clear();
+    CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  }
+  if (!graph) CK(cudaEventRecord(ev0, stream));
+  cudaError_t e = cudaSuccess;  // a failure inside a capture still ends the capture
+  if (!replay && (pc.useBias || dRef))
+    e = launch_planes_aux(d.bias, pc.biasShift, d.mult, pc.useBias ? biasP : nullptr, dRef ? multM : nullptr, ncol, stream);
+  if (!replay && e == cudaSuccess && dFinal) e = cudaMemsetAsync(dFinal, 0, (size_t)B * ncol * 4, stream);
+  if (!replay && e == cudaSuccess && dHist) e = cudaMemsetAsync(dHist, 0, (size_t)B * a.T * ncol * 4, stream);
+  for (uint32_t b0 = 0; !replay && b0 < B; b0 += Bc) {  // one launch per chunk of trajectories
+    PlanesDev r = d0;
+    c.B = std::min(Bc, B - b0);
+    r.stims = dCues + (size_t)b0 * ncol;
+    r.refBall = dRef ? dRef + (size_t)b0 * ncol : nullptr;
+    r.finalOut = dFinal ? dFinal + (size_t)b0 * ncol : nullptr;
+    r.hist = dHist ? dHist + (size_t)b0 * a.T * ncol : nullptr;
+    r.stats = dStats ? dStats + (size_t)b0 * 1024 : nullptr;
+    r.driveLog = dLog ? dLog + (size_t)b0 * 256 : nullptr;
+    const PlanesShape sh = planes_shape(ncol, c.B, sm_count, &c);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = planes_max_blocks_per_sm(c, sh, &per_sm);
+    if (e == cudaSuccess && per_sm < 1) e = cudaErrorInvalidConfiguration;
+    if (e == cudaSuccess) e = cudaMemsetAsync(zero, 0, zBytes, stream);
+    if (e == cudaSuccess) e = launch_recall_planes(r, c, sh, stream);
+    if (e != cudaSuccess) break;
+  }
+  if (graph && !replay) {
+    cudaGraph_t g = nullptr;
+    const cudaError_t ec = cudaStreamEndCapture(stream, &g);
+    if (e == cudaSuccess) e = ec;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&recallGraph, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+      recallGraph = nullptr;
+      return cuda_fail(e, "batched recall graph capture");
+    }
+    recallKey = key;
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "launch_recall_planes");
+  if (graph) {
+    CK(cudaEventRecord(ev0, stream));
+    CK(cudaGraphLaunch(recallGraph, stream));
+  }
+  CK(cudaEventRecord(ev1, stream));
+  return AXON_OK;
+}
 
 axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall_args& a, const uint32_t* refBall,
                              uint32_t* finalOut, uint32_t* hist, uint32_t* stats, uint32_t* driveLog, bool dev,
@@ -121,6 +238,9 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
       CK(launch_present(dd, pc, shape, stream));
     }
     CK(cudaEventRecord(ev1, stream));
+  } else if (planes_apply(cfg, a) && ensure_w3p() == AXON_OK) {
+    const axon_status st = recall_planes(dCues, B, a, dRef, dFinal, dHist, dStats, dLog);
+    if (st != AXON_OK) return st;
   } else {
     if (ncol > 8192) return set_error(AXON_EINVAL, "batched recall supports ncol <= 8192; use the plain method");
     axon_status st = ensure_w3b();

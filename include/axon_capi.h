@@ -181,17 +181,16 @@ typedef struct axon_recall_args {
                            captured CUDA graph, kept and replayed while every argument and
                            array stays the same (device-resident callers); 0 = launch directly */
   uint32_t contraction; /* batched method: the unit that computes k_drive's AND-popcounts
-                           (src/axon.mm:166-173): AXON_CONTRACT_POPC (0, __popc on the CUDA
-                           cores) or AXON_CONTRACT_TENSOR (1, binary MMA on the tensor cores);
+                           (src/axon.mm:166-173): AXON_CONTRACT_POPC (0, logic operations or __popc
+                           on the CUDA cores) or AXON_CONTRACT_TENSOR (1, binary MMA on the tensor cores);
                            the results are the same */
-  uint32_t slab;        /* batched method, 16-bit counters without bias or facilitation: which
-                           per-neuron drives the kernel stores for the k-of-32 of the columns
-                           that pass the gate. AXON_SLAB_FLOOR (0): those of columns whose
-                           drive reaches the trajectory's threshold-histogram floor (half its
-                           previous threshold), and every one at the step after the clamp;
-                           AXON_SLAB_FLOOR_ALWAYS (1): the floor at every step; AXON_SLAB_FULL
-                           (2): every one. A gated column without a stored drive has it
-                           recomputed; the results are the same */
+  uint32_t slab;        /* batched method: whose per-neuron drives the kernel keeps for the k-of-32 of the columns
+                           that pass the gate; the results are the same. AXON_SLAB_FLOOR (0): those of columns
+                           whose drive reaches a floor taken from the trajectory's earlier thresholds (with
+                           facilitation, drives of 2^14 and more, or the tensor contraction, half the previous one
+                           and every column at the step after the clamp); AXON_SLAB_FLOOR_ALWAYS (1): the same
+                           without a rule of its own for the step after the clamp; AXON_SLAB_FULL (2): every one.
+                           A gated column without a kept drive has it recomputed */
   uint32_t reserved[1]; /* zero */
 } axon_recall_args;
 

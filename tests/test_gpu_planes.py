@@ -1,0 +1,86 @@
+"""The bit-plane batched readout (lane = trajectory) against the plain path, at the edges of
+its cases: every form of spike-word record, both ways of reading the tiles, the lane split of
+small batches, more candidates and gated columns than a group's memory holds."""
+import numpy as np
+import pytest
+
+import axon_b200 as ax
+
+pytestmark = pytest.mark.gpu
+
+
+def trained(seed=0, nstim=6, epochs=3, **kw):
+    base = dict(ax.CONFIG_C, ncol=256, incols=64, target=16, k=12)
+    base.update(kw)
+    net = ax.Network(base)
+    net.init(seed)
+    stimcols = max(4, base["incols"] // 4)
+    pats = ax.stimuli(seed, nstim, base["incols"], stimcols)
+    for _ in range(epochs):
+        for p in range(nstim):
+            net.present(ax.load_stim(pats[p], 1.0, 1000 + p, net.ncol), 10, 5, True)
+    return net, pats
+
+
+def cues_of(net, pats, B, seed):
+    """Whole columns, dropped columns and single flipped bits: words of 1 to 32 set bits."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for b in range(B):
+        w = ax.clamp_words(pats[b % len(pats)], net.ncol)
+        keep = (1.0, 0.95, 0.7, 0.5, 0.3, 0.05)[b % 6]
+        if keep < 1.0:
+            bits = rng.random((net.ncol, 32)) < keep
+            w &= (bits.astype(np.uint64) << np.arange(32, dtype=np.uint64)).sum(1).astype(np.uint32)
+        out.append(w)
+    return np.stack(out)
+
+
+def same(net, cues, T, clamp, **kw):
+    a = net.recall(cues, T, clamp, hist=True, stats=True, **kw)
+    b = net.recall(cues, T, clamp, hist=True, stats=True, method="plain", **kw)
+    a["stats"][:, 2] = b["stats"][:, 2] = 0  # branch coincidence: plain method only
+    for k in ("final", "hist", "stats"):
+        assert np.array_equal(a[k], b[k]), k
+    if a["drive_log"] is not None:
+        assert np.array_equal(a["drive_log"], b["drive_log"])
+
+
+# winners per column: sums of the held or of the left-out neurons, of at most 8, 12 or 16 masks
+@pytest.mark.parametrize("k", [0, 1, 8, 12, 13, 16, 17, 19, 20, 23, 24, 31, 32, 40])
+def test_record_forms(k):
+    net, pats = trained(k=k)
+    same(net, cues_of(net, pats, 12, k), 16, 4)
+    net.close()
+
+
+@pytest.mark.parametrize("kw", [dict(dthr=3), dict(dthr=40), dict(dthr=600), dict(mode=0), dict(mode=2, dthr=2), dict(boost=255),
+                                dict(boost=77), dict(incols=20), dict(target=1), dict(target=250), dict(target=0),
+                                dict(target=0, topkpar=0)])
+@pytest.mark.parametrize("B", [9, 130])
+def test_dendrites_and_thresholds(kw, B):
+    net, pats = trained(**kw)
+    same(net, cues_of(net, pats, B, B), 14, 3)
+    same(net, cues_of(net, pats, B, B + 1), 14, 3, use_bias=1, slab="full")
+    net.close()
+
+
+# both sides of each line of the launch shape: lanes per trajectory, tiles through L2 or staged, one or more launches
+@pytest.mark.parametrize("B", [1, 10, 11, 20, 21, 32, 33, 96, 97, 160, 161, 296, 300, 512, 513])
+def test_batch_sizes(B):
+    net, pats = trained(ncol=608, incols=72, target=24, k=24)
+    same(net, cues_of(net, pats, B, B), 9, 3)
+    net.close()
+
+
+def test_wide_networks_with_logs():
+    """Several columns per slot and CTA at odd widths, more gated columns than the list holds
+    (target near ncol), and the drive log."""
+    rng = np.random.default_rng(5)
+    for ncol, B, kw in ((2080, 110, {}), (1984, 20, dict(target=1500)), (2208, 100, dict(target=1900)), (8192, 100, {})):
+        net, pats = trained(**dict(dict(ncol=ncol, incols=256, target=32, k=24, nstim=4, epochs=1), **kw))
+        net.write("MULT", rng.integers(0, 3, ncol * 32).astype(np.uint32))
+        ref = rng.integers(0, 1 << 32, (B, ncol), dtype=np.uint64).astype(np.uint32)
+        for slab in ("floor", "floor_always", "full"):
+            same(net, cues_of(net, pats, B, 3), 9, 3, ref_ball=ref if slab == "floor" else None, slab=slab)
+        net.close()
