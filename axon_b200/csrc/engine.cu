@@ -71,7 +71,7 @@ axon_status pick_present_shape(uint32_t ncol, uint32_t incols, int sms, LaunchSh
     const int grid = (int)((warps + wpb - 1) / wpb);
     const size_t smem = present_smem_bytes(ncol, incols, cpw);
     int per_sm = 0;
-    CK(present_max_blocks_per_sm(cpw, wpb * 32, smem, &per_sm));
+    CK(present_max_blocks_per_sm(cpw, (int)kPresentMaxWarps * 32, smem, &per_sm));  // learning launches take full CTAs
     if (per_sm >= 1 && grid <= per_sm * sms) {
       out->cpw = cpw;
       out->wpb = wpb;

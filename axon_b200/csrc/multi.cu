@@ -314,14 +314,15 @@ __global__ void __launch_bounds__(NT, 1) k_multi(MultiDev m, MultiCfg c) {
                   p2[jj] = __ldcg(P2 + base4 + 32 * jj);
                   p3[jj] = __ldcg(P3 + base4 + 32 * jj);
                 }
+                const Band band = band_of(c.bandLo, c.bandHi);
                 uint32_t nLTP = 0, nLTD = 0;
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {
                   const uint4 sp4 = sIn4[2 * g + jj];
-                  learn_word(p0[jj].x, p1[jj].x, p2[jj].x, p3[jj].x, sp4.x, want, phase, t, c, nLTP, nLTD);
-                  learn_word(p0[jj].y, p1[jj].y, p2[jj].y, p3[jj].y, sp4.y, want, phase, t, c, nLTP, nLTD);
-                  learn_word(p0[jj].z, p1[jj].z, p2[jj].z, p3[jj].z, sp4.z, want, phase, t, c, nLTP, nLTD);
-                  learn_word(p0[jj].w, p1[jj].w, p2[jj].w, p3[jj].w, sp4.w, want, phase, t, c, nLTP, nLTD);
+                  learn_word(p0[jj].x, p1[jj].x, p2[jj].x, p3[jj].x, sp4.x, want, phase, t, c, band, nLTP, nLTD);
+                  learn_word(p0[jj].y, p1[jj].y, p2[jj].y, p3[jj].y, sp4.y, want, phase, t, c, band, nLTP, nLTD);
+                  learn_word(p0[jj].z, p1[jj].z, p2[jj].z, p3[jj].z, sp4.z, want, phase, t, c, band, nLTP, nLTD);
+                  learn_word(p0[jj].w, p1[jj].w, p2[jj].w, p3[jj].w, sp4.w, want, phase, t, c, band, nLTP, nLTD);
                 }
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {

@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, 
   const uint32_t ncol = c.ncol, incols = c.incols;
   const uint32_t ngrp = ncol / 8u, nactw = (((ngrp + 31u) / 32u) + 3u) & ~3u;  // 16-byte multiple
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, wpb = blockDim.x >> 5;
-  const uint32_t maxCols = wpb * CPW;      // columns owned by this CTA
+  const uint32_t own = c.ownWarps;         // the warps that own columns; the others help with copies and learning
+  const uint32_t maxCols = own * CPW;      // columns owned by this CTA
   const PresentSmem L = present_smem_layout(ncol, incols, CPW);
   uint32_t* sSpk0 = sm;                    // spike vectors, ping-pong
   uint32_t* sSpk1 = sm + ncol;
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, 
   // columns are dealt to warps CTA-interleaved (column = warp * grid + CTA): the clamped
   // input columns, which all fire and learn during the clamp, spread over every CTA instead
   // of loading the first few
-  const uint32_t gwarp = warp * gridDim.x + blockIdx.x, nwarps = gridDim.x * wpb;
+  const uint32_t gwarp = warp < own ? warp * gridDim.x + blockIdx.x : ncol, nwarps = gridDim.x * own;
   uint32_t* xhist = d.bar + 64;            // step t counts its recurrent drives into histogram t mod 3
   // branch term of k_drive (src/axon.mm:174-178): the count (modes 0, 1) plus, when the
   // branch reaches dthr, the boost (mode 1) or 1 (mode 2)
@@ -352,14 +353,15 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, 
           p2[j] = __ldcg(d.W2 + base + 32 * j);
           p3[j] = __ldcg(d.W3 + base + 32 * j);
         }
+        const Band band = band_of(c.bandLo, c.bandHi);
         uint32_t nLTP = 0, nLTD = 0;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const uint4 sp4 = sIn4[2 * g + j];
-          learn_word(p0[j].x, p1[j].x, p2[j].x, p3[j].x, sp4.x, want, phase, t, c, nLTP, nLTD);
-          learn_word(p0[j].y, p1[j].y, p2[j].y, p3[j].y, sp4.y, want, phase, t, c, nLTP, nLTD);
-          learn_word(p0[j].z, p1[j].z, p2[j].z, p3[j].z, sp4.z, want, phase, t, c, nLTP, nLTD);
-          learn_word(p0[j].w, p1[j].w, p2[j].w, p3[j].w, sp4.w, want, phase, t, c, nLTP, nLTD);
+          learn_word(p0[j].x, p1[j].x, p2[j].x, p3[j].x, sp4.x, want, phase, t, c, band, nLTP, nLTD);
+          learn_word(p0[j].y, p1[j].y, p2[j].y, p3[j].y, sp4.y, want, phase, t, c, band, nLTP, nLTD);
+          learn_word(p0[j].z, p1[j].z, p2[j].z, p3[j].z, sp4.z, want, phase, t, c, band, nLTP, nLTD);
+          learn_word(p0[j].w, p1[j].w, p2[j].w, p3[j].w, sp4.w, want, phase, t, c, band, nLTP, nLTD);
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, 
 #pragma unroll
       for (int i = 0; i < CPW; ++i) {
         const uint32_t slot = warp * CPW + (uint32_t)i;
-        if (col[i] >= ncol || sMark[slot] != t + 1u) continue;
+        if (col[i] >= ncol || sMark[slot] != t + 1u) continue;  // (helper warps own no column)
         const uint32_t nLTP = sLTP[slot * 32u + lane], nLTD = sLTD[slot * 32u + lane];
         const uint32_t sumP = __reduce_add_sync(kFull, nLTP), sumD = __reduce_add_sync(kFull, nLTD);
         const uint32_t kP = __popc(__ballot_sync(kFull, nLTP != 0u)), kD = __popc(__ballot_sync(kFull, nLTD != 0u));
@@ -430,14 +432,21 @@ static const void* present_fn(int cpw, bool learn) {
   }
 }
 
-cudaError_t launch_present(const NetDev& d, const PresentCfg& c, const LaunchShape& ls, cudaStream_t st) {
+cudaError_t launch_present(const NetDev& d, const PresentCfg& cfg, const LaunchShape& ls, cudaStream_t st) {
+  PresentCfg c = cfg;
+  c.ownWarps = (uint32_t)ls.wpb;
+  // Learning takes a full CTA: a firing column's voted branches (up to 32 updates of 8 KiB)
+  // run one per warp at a time, and the CTAs with most of them hold up the grid barrier.
+  // With the owners alone (2 warps a CTA at 256 columns, 7 at 1,024, 15 at 2,080) a 10-step
+  // presentation took 170 / 121 / 131 us, with full CTAs 108 / 108 / 125.
+  const int warps = c.learn ? (int)kPresentMaxWarps : ls.wpb;
   void* args[] = {(void*)&d, (void*)&c};
   const void* fn = present_fn(ls.cpw, c.learn != 0u);
   if (!fn) return cudaErrorInvalidValue;
   // barrier counter and the three drive histograms start at zero
   const cudaError_t e = cudaMemsetAsync(d.bar, 0, kBarRegionWords * 4u, st);
   if (e != cudaSuccess) return e;
-  return cudaLaunchCooperativeKernel(fn, dim3(ls.grid), dim3(ls.wpb * 32), args, ls.smem, st);
+  return cudaLaunchCooperativeKernel(fn, dim3(ls.grid), dim3(warps * 32), args, ls.smem, st);
 }
 
 // Sets the shared-memory size of both forms (learning, readout) and returns the smaller

@@ -55,13 +55,14 @@ __host__ __device__ inline PresentSmem present_smem_layout(uint32_t ncol, uint32
 struct PresentCfg {
   uint32_t ncol, incols, T, clampSteps, learn, k, dthr, boost, mode, targetCols, useBias, facil, biasUp, biasDown,
       biasShift, biasDownEvery, bandLo, bandHi, marginGate, hetero, ltdRep, contrast, ltdEvery, topkPar;
+  uint32_t ownWarps; // warps per CTA that own columns (set by launch_present)
   uint32_t missing;  // CTAs every grid barrier waits for beyond the launch: 0, or more to test failure detection
   uint64_t waitNs;
 };
 
 struct LaunchShape {
   int cpw;       // columns per warp (1, 2)
-  int wpb;       // warps per block
+  int wpb;       // warps per block that own columns
   int grid;      // blocks (all co-resident)
   size_t smem;   // dynamic shared memory bytes
 };
