@@ -20,6 +20,7 @@
 #include "emit.cuh"
 #include "learn.cuh"
 #include "multi.cuh"
+#include "present.cuh"
 #include "theta.cuh"
 
 namespace axon {
@@ -401,20 +402,107 @@ __global__ void __launch_bounds__(NT, 1) k_multi(MultiDev m, MultiCfg c) {
   if (lane == 0 && nTiles) atomicAdd(m.work, (unsigned long long)nTiles);
 }
 
+// Slots of enough CTAs that a warp owns at most CPW = 1 or 2 columns: the plain kernel's step
+// loop (present.cuh: tiles of all the CTA's columns in flight in a shared-memory pool,
+// threshold from the published drive histogram, per-neuron state on chip), each slot running
+// its queue of networks and their programs. In the register form such a slot's step is a
+// chain of L2 round trips. Launch time, register form / pool (the tuner takes the faster):
+// one network of 256 columns 16.1 / 12.9 ms, three of 640 28.2 / 24.7 ms, four of 1,056 36.8 /
+// 28.5 ms; from 2,080 columns on the two are level (26.3 / 26.4 ms for two networks).
+template <int CPW>
+__global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_multi_pool(MultiDev m, MultiCfg c) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  uint32_t slot = 0;
+  while (slot + 1u < m.nslots && blockIdx.x >= m.slots[slot + 1u].cta0) ++slot;
+  const MultiSlot S = m.slots[slot];
+  if (blockIdx.x < S.cta0 || blockIdx.x >= S.cta0 + S.ncta) return;  // not covered (the host never does this)
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const PresentSmem L = present_smem_layout(c.ncol, c.incols, CPW);
+  const PresentTeam tm{blockIdx.x - S.cta0, S.ncta, (c.ncol + S.ncta * CPW - 1u) / (S.ncta * CPW), L.poolTiles - 1u,
+                       m.bars + slot * 32u, m.hist + (size_t)slot * 3u * kHistWords};
+  // the pool's last tile holds the network's pointers and the presentation's parameters
+  NetDev* sNet = reinterpret_cast<NetDev*>(sm + L.poolWord + (L.poolTiles - 1u) * 256u);
+  PresentCfg* sCfg = reinterpret_cast<PresentCfg*>(sNet + 1);
+  static_assert(sizeof(NetDev) + sizeof(PresentCfg) <= 1024u, "the two structures share one tile");
+  PresentCta<CPW> w;
+  w.init(sm, c.ncol, c.incols, tm);
+  if (tid == 0) {
+    PresentCfg p{};
+    p.ncol = c.ncol; p.incols = c.incols; p.dthr = c.dthr; p.boost = c.boost; p.mode = c.mode;
+    p.targetCols = c.targetCols; p.biasUp = c.biasUp; p.biasDown = c.biasDown; p.biasShift = c.biasShift;
+    p.biasDownEvery = c.biasDownEvery; p.bandLo = c.bandLo; p.bandHi = c.bandHi; p.marginGate = c.marginGate;
+    p.hetero = c.hetero; p.ltdRep = c.ltdRep; p.contrast = c.contrast; p.ltdEvery = c.ltdEvery; p.topkPar = c.topkPar;
+    p.ownWarps = tm.own; p.missing = c.missing; p.waitNs = c.waitNs;
+    *sCfg = p;
+  }
+  uint32_t g = 0;  // steps the slot has run
+  for (uint32_t qi = S.q0; qi < S.q1; ++qi) {
+    const MultiNet* N = m.nets + m.queue[qi];
+    const uint32_t nprog = N->nprog;
+    __syncthreads();
+    if (tid == 0) {
+      *sNet = N->d;
+      sNet->err = m.err;
+    }
+    __syncthreads();
+    w.load(*sNet);
+    bool learned = false;
+    for (uint32_t pi = 0; pi < nprog; ++pi) {
+      if (tid == 0) {
+        const MultiPresent p = N->prog[pi];
+        sNet->stim = const_cast<uint32_t*>(p.stim);
+        sNet->refBall = const_cast<uint32_t*>(p.refBall);
+        sNet->hist = p.hist;
+        sNet->finalOut = p.finalOut;
+        sNet->stats = p.stats;
+        sNet->driveLog = p.driveLog;
+        sCfg->T = p.T; sCfg->clampSteps = p.clampSteps; sCfg->learn = p.learn; sCfg->useBias = p.useBias;
+        sCfg->k = p.k; sCfg->facil = p.facil;
+      }
+      __syncthreads();
+      w.begin(*sNet);
+      __syncthreads();
+      const bool learn = sCfg->learn != 0u;
+      if (!(learn ? w.template steps<true>(*sNet, *sCfg, tm, g) : w.template steps<false>(*sNet, *sCfg, tm, g))) return;
+      w.end(*sNet, sCfg->T);
+      g += sCfg->T;
+      learned = learned || learn;
+      __syncthreads();
+    }
+    if (learned) w.store_bias(*sNet);
+  }
+  if (lane == 0 && w.nTiles) atomicAdd(m.work, (unsigned long long)w.nTiles);
+  if (tid == 0 && w.nTasks) atomicAdd(m.work + 1, (unsigned long long)w.nTasks);
+}
+
 // ---------------------------------------------------------------- launch helpers
+// columns per warp of the pool form when the smallest slot has ncta CTAs, 0 when it does not fit
+int multi_pool_cpw(uint32_t ncol, uint32_t incols, uint32_t ncta) {
+  for (int cpw : {1, 2}) {
+    const PresentSmem L = present_smem_layout(ncol, incols, cpw);
+    if (ncta * kPresentMaxWarps * (uint32_t)cpw >= ncol && L.bytes <= kSmemLimitBytes &&
+        (L.poolTiles - 1u) * 256u >= 3u * ncol)
+      return cpw;
+  }
+  return 0;
+}
+
+static const void* pool_fn(int cpw) { return cpw == 1 ? (const void*)k_multi_pool<1> : (const void*)k_multi_pool<2>; }
+
 size_t multi_smem_bytes(uint32_t ncol, uint32_t incols, uint32_t maxCpw, int threads) {
   return (size_t)multi_layout(ncol, incols, (uint32_t)(threads / 32) * maxCpw).total * 4;
 }
 
-static const void* multi_fn(int threads, int tiles) {
+static const void* multi_fn(int threads, int tiles, int cpw) {
+  if (tiles == 0) return pool_fn(cpw);
   if (threads == 1024 && tiles == 4) return (const void*)k_multi<1024, 4>;
   if (threads == 896 && tiles == 4) return (const void*)k_multi<896, 4>;
   if (threads == 512 && tiles == 8) return (const void*)k_multi<512, 8>;
   return nullptr;
 }
 
-cudaError_t multi_max_blocks_per_sm(int threads, int tiles, size_t smem, int* out) {
-  const void* fn = multi_fn(threads, tiles);
+cudaError_t multi_max_blocks_per_sm(int threads, int tiles, int cpw, size_t smem, int* out) {
+  const void* fn = multi_fn(threads, tiles, cpw);
   if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -422,7 +510,7 @@ cudaError_t multi_max_blocks_per_sm(int threads, int tiles, size_t smem, int* ou
 }
 
 cudaError_t launch_multi(const MultiDev& m, const MultiCfg& c, const MultiShape& s, cudaStream_t st) {
-  const void* fn = multi_fn(s.threads, s.tiles);
+  const void* fn = multi_fn(s.threads, s.tiles, s.cpw);
   if (!fn) return cudaErrorInvalidValue;
   void* args[] = {(void*)&m, (void*)&c};
   return cudaLaunchCooperativeKernel(fn, dim3(s.grid), dim3(s.threads), args, s.smem, st);

@@ -39,6 +39,7 @@ struct MultiDev {
   const MultiNet* nets;
   const MultiSlot* slots;   // sorted by cta0, covering the whole grid
   const uint32_t* queue;    // network indices, grouped by slot
+  uint32_t* hist;           // [nslots][3 * kHistWords] drive histograms (pool form), zeroed
   uint32_t* bars;           // [nslots * 32] barrier counters (one 128-byte line each), zeroed
   uint32_t* err;            // device error word
   unsigned long long* work; // [0] W3 tiles read by the drive, [1] learning tasks (branch read-modify-writes)
@@ -54,15 +55,16 @@ struct MultiCfg {
   uint64_t waitNs;
 };
 
-// Launch shape: (threads, tiles) is (1024, 4), (896, 4) or (512, 8), one CTA per SM;
-// grid = CTAs of all slots.
+// Launch shape: (threads, tiles) is (1024, 4), (896, 4) or (512, 8), or (896, 0) for the pool
+// form with cpw columns per warp; one CTA per SM; grid = CTAs of all slots.
 struct MultiShape {
-  int threads, tiles, grid;
+  int threads, tiles, grid, cpw;
   size_t smem;
 };
 
 size_t multi_smem_bytes(uint32_t ncol, uint32_t incols, uint32_t maxCpw, int threads);
-cudaError_t multi_max_blocks_per_sm(int threads, int tiles, size_t smem, int* out);
+int multi_pool_cpw(uint32_t ncol, uint32_t incols, uint32_t ncta);
+cudaError_t multi_max_blocks_per_sm(int threads, int tiles, int cpw, size_t smem, int* out);
 cudaError_t launch_multi(const MultiDev& m, const MultiCfg& c, const MultiShape& s, cudaStream_t st);
 
 }  // namespace axon

@@ -139,7 +139,8 @@ class MultiRun {
   size_t offQueue() const { return offSlots() + al(kMaxSlots * sizeof(MultiSlot)); }
   size_t offBars() const { return offQueue() + al(n_ * 4); }
   size_t offErr() const { return offBars() + al(kMaxSlots * 32 * 4); }
-  size_t offHist() const { return offErr() + al(64); }
+  size_t offTh() const { return offErr() + al(64); }  // per slot of the pool form (at most one per SM)
+  size_t offHist() const { return offTh() + al((size_t)net0_->sm_count * 3 * kHistWords * 4); }
   size_t offStats() const { return offHist() + al((size_t)64 * ncol_ * 4); }
   size_t offDlog() const { return offStats() + al(1024 * 4); }
   size_t offZeros() const { return offDlog() + al(256 * 4); }
@@ -293,20 +294,29 @@ axon_status MultiRun::launch(const Shape& sh, const std::vector<std::vector<uint
   m.err = dErr;
   m.work = reinterpret_cast<unsigned long long*>(dErr + 4);  // 16 bytes into the error word's 64-byte line
   m.nslots = S;
+  m.hist = (uint32_t*)(ctl + offTh());
   MultiCfg c = cfg_;
   c.maxCpw = max_cpw(ncta, sh.threads);
   MultiShape shp{};
   shp.threads = sh.threads;
   shp.tiles = sh.tiles;
   shp.grid = (int)cta;
-  shp.smem = multi_smem_bytes(ncol_, incols_, c.maxCpw, sh.threads);
+  const bool pool = sh.tiles == 0;
+  if (pool) {
+    shp.cpw = multi_pool_cpw(ncol_, incols_, *std::min_element(ncta.begin(), ncta.end()));
+    if (shp.cpw == 0 || S > (uint32_t)net0_->sm_count) return set_error(AXON_EINVAL, "multi-network shape does not fit the GPU");
+    shp.smem = present_smem_bytes(ncol_, incols_, shp.cpw);
+  } else {
+    shp.smem = multi_smem_bytes(ncol_, incols_, c.maxCpw, sh.threads);
+  }
   int per = 0;
-  CK(multi_max_blocks_per_sm(sh.threads, sh.tiles, shp.smem, &per));
+  CK(multi_max_blocks_per_sm(sh.threads, sh.tiles, shp.cpw, shp.smem, &per));
   if (per < 1 || (int)cta > per * net0_->sm_count) return set_error(AXON_EINVAL, "multi-network shape does not fit the GPU");
 
   auto body = [&]() -> cudaError_t {
     cudaError_t e = cudaMemsetAsync(dBars, 0, (size_t)S * 32 * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(dErr, 0, 32, st);  // error word and work counters
+    if (e == cudaSuccess && pool) e = cudaMemsetAsync(m.hist, 0, (size_t)S * 3 * kHistWords * 4, st);
     if (e == cudaSuccess) e = launch_multi(m, c, shp, st);
     return e;
   };
@@ -396,7 +406,7 @@ axon_status MultiRun::tune(Shape* best, std::vector<std::vector<uint32_t>>* best
   std::vector<uint64_t> cost(n_);
   for (uint32_t i = 0; i < n_; ++i) cost[i] = plans_[i].steps;
   const uint32_t slotCands[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 25, 32, 40, 50, 64, 74};
-  const int shapeCands[][2] = {{1024, 4}, {896, 4}, {512, 8}};
+  const int shapeCands[][2] = {{896, 0}, {1024, 4}, {896, 4}, {512, 8}};
   double bestT = 1e300;
   *tuneMs = 0.f;
   *tried = 0;
@@ -404,7 +414,9 @@ axon_status MultiRun::tune(Shape* best, std::vector<std::vector<uint32_t>>* best
     for (uint32_t S : slotCands) {
       if (S > n_ || S > grid) continue;
       const std::vector<uint32_t> ncta = split_ctas(grid, S);
-      if (multi_smem_bytes(ncol_, incols_, max_cpw(ncta, sc[0]), sc[0]) > 227 * 1024) continue;
+      if (sc[1] == 0 ? multi_pool_cpw(ncol_, incols_, *std::min_element(ncta.begin(), ncta.end())) == 0
+                     : multi_smem_bytes(ncol_, incols_, max_cpw(ncta, sc[0]), sc[0]) > 227 * 1024)
+        continue;
       // calibration: slot s runs network s for a few learning presentations
       std::vector<std::vector<uint32_t>> q(S);
       std::vector<uint32_t> np(n_, 0u);
@@ -565,6 +577,10 @@ axon_status MultiRun::run(const uint32_t* seeds, const uint32_t* nstim, axon_mul
       sh.tiles = sh.threads == 512 ? 8 : 4;
       if (sh.slots > (uint32_t)net0_->sm_count) return set_error(AXON_EINVAL, "more slots than SMs");
       ncta = split_ctas((uint32_t)net0_->sm_count, sh.slots);
+      if (a_.threads == 0 && multi_pool_cpw(ncol_, incols_, *std::min_element(ncta.begin(), ncta.end()))) {
+        sh.threads = (int)kPresentMaxWarps * 32;
+        sh.tiles = 0;
+      }
       std::vector<uint64_t> cost(n_);
       for (uint32_t i = 0; i < n_; ++i) cost[i] = plans_[i].steps;
       assign(cost, ncta, queues);

@@ -273,7 +273,8 @@ typedef struct axon_multi_args {
   uint32_t readout;     /* 1: run the readouts and fill results */
   uint32_t autotune;    /* 1: pick slots and CTA shape by timing candidates */
   uint32_t slots;       /* autotune == 0: concurrent networks (0 = one per network, at most one per SM) */
-  uint32_t threads;     /* autotune == 0: 1024 or 896 (4 W3 tiles in flight per warp) or 512 (8 tiles) */
+  uint32_t threads;     /* autotune == 0: 1024 or 896 (4 W3 tiles in flight per warp) or 512 (8 tiles); 0 = tiles in a
+                           shared-memory pool (896 threads) when a warp owns at most 2 columns, else 1024 */
   uint32_t graph;       /* 1: launch through a captured CUDA graph */
   uint32_t method;      /* 0: one persistent launch, 1: plain path, one launch per presentation */
   uint32_t reserved[4]; /* zero */
@@ -295,7 +296,7 @@ typedef struct axon_multi_report {
   double tune_ms;       /* device time spent timing candidate shapes */
   uint64_t steps;       /* network-steps run */
   uint64_t train_steps; /* of which learning steps */
-  uint32_t slots, threads, tiles, grid; /* shape used (slots = 0 for the plain path) */
+  uint32_t slots, threads, tiles, grid; /* shape used (slots = 0 for the plain path, tiles = 0 for the tile pool) */
   uint32_t graph;       /* 1 when the launch ran as a CUDA graph */
   uint32_t tried;       /* candidate shapes timed */
   uint64_t w3_tiles;    /* W3 tiles (1 KiB each) the drive read: (column, branch) pairs with a spiking group */
