@@ -18,29 +18,60 @@ constexpr uint32_t kPlanes = 14;                    // bit planes of a per-neuro
 constexpr uint32_t kPlanesMaxB = 512;               // trajectories per launch (the host splits larger batches)
 constexpr uint32_t kPlanesVals = 1536;              // candidates a phase-2 group keeps in shared memory
 constexpr uint32_t kPlanesList = 512;               // gated columns it lists there
-constexpr uint32_t kPlanesThreads = 640;  // 96 registers: no spills in phase 1
+// 640 threads leave 96 registers; tiles read through L2 want more warps (at most 28: a phase-2
+// group keeps two words per warp beside its counters)
+constexpr int planes_threads(bool direct) { return direct ? 896 : 640; }
+
+constexpr uint32_t kPlanesDirectB = 160;            // most trajectories whose tiles are read through L2
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
+
+// A network and the team's words for it.
+struct PlanesNet {
+  const uint32_t* W3P;    // [ncol][kPlaneCol]
+  const uint32_t* conn;   // [ncol*32]
+  uint32_t* act;          // [2][ngrp][astr] by step parity: bit j of word (g, k) = trajectory 32k + j spikes in group g
+  uint32_t* bar;          // grid barrier counter (zeroed before the launch)
+  const uint32_t* lanes;  // server: entry of each trajectory, or kNoSlot
+  uint32_t astr, par;     // words per group of act; its parity that the launch's first step reads
+};
+
+// The server's tables: the CTAs and trajectories of one network, and one trajectory.
+struct PlanesTeam {
+  PlanesNet net;
+  uint32_t cta0, ncta, B;
+};
+struct PlanesEntry {
+  uint32_t slot;             // state slot
+  uint32_t t0, clamp, steps;  // its step at the launch's first, clamped steps, all steps
+  uint32_t ncue, cueOff;     // clamped input columns, in the launch's cue area
+  uint32_t done;             // row of its final spikes when it ends in this launch
+  uint32_t pad;
+};
 
 struct PlanesDev {
-  const uint32_t* W3P;      // [ncol][kPlaneCol]
-  const uint32_t* conn;     // [ncol*32]
+  PlanesNet net;            // (the server takes the team's)
   const uint32_t* biasP;    // [ncol][16] planes of min(bias >> shift, 2^14 - 1), or null (no bias)
   const uint32_t* multM;    // [ncol] neurons with multiplicity > 1 (with refBall)
   const uint32_t* stims;    // [B][ncol] clamp patterns
   const uint32_t* refBall;  // [B][ncol] logged reference assemblies, or null
-  uint32_t* act;            // [2][ngrp][nblk] by step parity: bit j of word (g, k) = trajectory 32k + j spikes in group g
   uint4* rec;               // [B][ngrp + ncol] per group the record of its first nonzero spike word, then per
                             // column the records of the further ones
-  uint32_t* drv;            // [ncol][32 * nblk] column drives of the step
   uint32_t* candB;          // [B][ncol/32] candidates of the step, a bit per column (zeroed before the launch)
-  uint4* candP;             // [B][ncol][4] their drive planes (words 0..13) and column drives (word 14)
-  uint32_t* ball;           // [B][ncol] ballots of a step with more than kPlanesList gated columns
-  uint32_t* thPrev;         // [2][B] the last two thresholds, by step parity
+  uint4* candP;             // [B][ncol][4] their drive planes (words 0..13); word 15: the ballot, in a step with more
+                            // than kPlanesList gated columns
+  uint32_t* drv;            // column drives of the step, trajectory b's column c at b * drvB + c * drvC
+  uint32_t* thPrev;         // [2][thStride] the last two thresholds, by step parity
   uint32_t* finalOut;       // [B][ncol] spikes of the last step (zeroed before the launch), or null
   uint32_t* hist;           // [B][T][ncol] spikes of every step (zeroed before the launch), or null
   uint32_t* stats;          // [B][1024] counters (zeroed before the launch), or null
   uint32_t* driveLog;       // [B][256] member-drive log (accumulated), or null
-  uint32_t* bar;            // grid barrier counter
   uint32_t* err;            // device error word
+  uint32_t drvB, drvC, thStride;
+  // server (B counts state slots above): finalOut holds the rows of the trajectories that end
+  const PlanesTeam* teams;  // by cta0, covering the grid
+  const PlanesEntry* entries;
+  const uint32_t* cues;
+  uint32_t nteams;
 };
 
 struct PlanesCfg {
@@ -64,6 +95,11 @@ struct PlanesShape {
 PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c);
 cudaError_t planes_max_blocks_per_sm(const PlanesCfg& c, const PlanesShape& s, int* out);
 cudaError_t launch_recall_planes(const PlanesDev& d, const PlanesCfg& c, const PlanesShape& s, cudaStream_t st);
+// The server's form: at most B trajectories in a team and `cols` columns in a CTA, `want`
+// phase-2 groups; fills the last fields of c.
+PlanesShape planes_serve_shape(uint32_t ncol, uint32_t B, int grid, uint32_t cols, uint32_t want, PlanesCfg* c);
+cudaError_t planes_serve_prepare(const PlanesCfg& c);
+cudaError_t launch_serve_planes(const PlanesDev& d, const PlanesCfg& c, const PlanesShape& s, cudaStream_t st);
 // W3 [col][s][j][lane][comp] -> W3P
 cudaError_t launch_make_w3p(const uint4* W3, uint32_t* W3P, uint32_t ncol, cudaStream_t st);
 // bias planes and multiplicity masks (either output may be null)

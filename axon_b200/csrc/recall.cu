@@ -65,14 +65,10 @@ namespace {
 size_t al(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 }  // namespace
 
-namespace {
-// The bit-plane kernel takes readouts whose per-neuron drives stay below 2^14 (drive << 13 |
-// column fits one word), without facilitation and on the CUDA cores.
-bool planes_apply(const axon_cfg& cfg, const axon_recall_args& a) {
+bool axon::planes_config(const axon_cfg& cfg) {
   const uint64_t maxAcc = cfg.mode == 2 ? 32ull : 32ull * (256ull + (cfg.mode == 1 ? cfg.boost : 0u));
-  return a.contraction == AXON_CONTRACT_POPC && cfg.facil == 0u && maxAcc < (1ull << kPlanes) && cfg.ncol <= 8192u;
+  return cfg.facil == 0u && maxAcc < (1ull << kPlanes) && cfg.ncol <= 8192u;
 }
-}  // namespace
 
 axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
                                     uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog) {
@@ -89,26 +85,25 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   // zeroed before every launch: activity words of both parities, candidate bits, thresholds,
   // the barrier word
   const size_t zBytes = al(2ull * ngrp * nblk * 4) + al((size_t)Bc * (ncol / 32u) * 4) + al((size_t)Bc * 8) + 256;
-  const size_t need = zBytes + al((size_t)Bc * (ngrp + ncol) * 16) + al((size_t)ncol * nblk * 32 * 4) +
-                      al(bnc * 64) + al(bnc * 4) + al((size_t)ncol * 64) + al((size_t)ncol * 4);
+  const size_t need = zBytes + al((size_t)Bc * (ngrp + ncol) * 16) + al((size_t)ncol * nblk * 32 * 4) + al(bnc * 64) +
+                      al((size_t)ncol * 64) + al((size_t)ncol * 4);
   axon_status st = scratch.ensure(need);
   if (st != AXON_OK) return st;
   char* p = (char*)scratch.p;
   auto take = [&](size_t bytes) { char* r = p; p += al(bytes); return r; };
   PlanesDev d0{};
   char* zero = p;
-  d0.act = (uint32_t*)take(2ull * ngrp * nblk * 4);
+  d0.net.act = (uint32_t*)take(2ull * ngrp * nblk * 4);
   d0.candB = (uint32_t*)take((size_t)Bc * (ncol / 32u) * 4);
   d0.thPrev = (uint32_t*)take((size_t)Bc * 8);
-  d0.bar = (uint32_t*)take(256);
+  d0.net.bar = (uint32_t*)take(256);
   d0.rec = (uint4*)take((size_t)Bc * (ngrp + ncol) * 16);
   d0.drv = (uint32_t*)take((size_t)ncol * nblk * 32 * 4);
   d0.candP = (uint4*)take(bnc * 64);
-  d0.ball = (uint32_t*)take(bnc * 4);
   uint32_t* biasP = (uint32_t*)take((size_t)ncol * 64);
   uint32_t* multM = (uint32_t*)take((size_t)ncol * 4);
-  d0.W3P = w3p;
-  d0.conn = d.conn;
+  d0.net.W3P = w3p;
+  d0.net.conn = d.conn;
   d0.biasP = pc.useBias ? biasP : nullptr;
   d0.multM = multM;
   d0.err = d.err;
@@ -133,6 +128,10 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   for (uint32_t b0 = 0; !replay && b0 < B; b0 += Bc) {  // one launch per chunk of trajectories
     PlanesDev r = d0;
     c.B = std::min(Bc, B - b0);
+    r.net.astr = (c.B + 31u) / 32u;
+    r.drvB = 1u;
+    r.drvC = 32u * r.net.astr;
+    r.thStride = c.B;
     r.stims = dCues + (size_t)b0 * ncol;
     r.refBall = dRef ? dRef + (size_t)b0 * ncol : nullptr;
     r.finalOut = dFinal ? dFinal + (size_t)b0 * ncol : nullptr;
@@ -238,7 +237,7 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
       CK(launch_present(dd, pc, shape, stream));
     }
     CK(cudaEventRecord(ev1, stream));
-  } else if (planes_apply(cfg, a) && ensure_w3p() == AXON_OK) {
+  } else if (a.contraction == AXON_CONTRACT_POPC && planes_config(cfg) && ensure_w3p() == AXON_OK) {
     const axon_status st = recall_planes(dCues, B, a, dRef, dFinal, dHist, dStats, dLog);
     if (st != AXON_OK) return st;
   } else {

@@ -40,8 +40,11 @@ struct Request {
 struct Active {
   uint32_t slot;
   uint32_t tloc;
+  uint32_t lane;  // bit-plane form: the trajectory's lane of its network, kept for its life
   Request req;
 };
+
+constexpr uint32_t kServeSteps = 8;  // most steps of one launch (bit-plane form)
 
 struct Done {
   axon_serve_result r;
@@ -97,12 +100,27 @@ struct axon_server {
   // the previous tick, until its results are retired
   std::vector<Finished> pending;
   bool pendingTick = false;
-  uint32_t pendingNe = 0, pendingEv = 0;
+  uint32_t pendingNe = 0, pendingEv = 0, pendingSteps = 1;
   size_t nRunning = 0;  // trajectories in the tables (nActive also counts those not yet retired)
 
+  // bit-plane form (planes_kernel.cuh): one launch advances every trajectory by one or more steps
+  bool planes = false;
+  PlanesDev pdev{};
+  PlanesCfg pcfg{};
+  uint32_t* actMem = nullptr;                   // activity words, [net][2][ngrp][kServeMaxB / 32]
+  std::vector<uint32_t> netPar;                 // per network: parity that its next step reads
+  std::vector<std::vector<uint32_t>> laneUsed;  // per network: bitmap of the lanes in use
+  std::vector<PlanesEntry> pentH;
+  std::vector<PlanesTeam> teamH;
+  std::vector<uint32_t> laneH;
+  double stepS = 0;  // wall time per step of the last launch
+
   axon_status start(axon_net* const* ns, uint32_t n, uint64_t memBytes);
+  axon_status start_planes(uint64_t memBytes);
   void loop();
+  void admit();
   axon_status tick();
+  axon_status tick_planes();
   axon_status retire_pending();
   void fail(axon_status s, const std::string& m) {
     std::lock_guard<std::mutex> g(mu);
@@ -143,6 +161,13 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
   const uint32_t packed = (!cfg.acc32 && cfg.facil == 0u) ? 1u : 0u;
   capB = packed ? kServeMaxB : kServeMaxB32;
   CKS(cudaSetDevice(device));
+  // the bit-plane form where it applies and its layout fits the device's memory
+  planes = planes_config(n0->cfg) && n <= (uint32_t)sms;
+  for (uint32_t i = 0; planes && i < n; ++i) {
+    planes = nets[i]->ensure_w3p() == AXON_OK;
+    if (planes) CKS(cudaStreamSynchronize(nets[i]->stream));
+  }
+  if (planes) return start_planes(memBytes);
   for (axon_net* x : nets) {  // the batched tile layout of every served network
     axon_status st = x->ensure_w3b();
     if (st != AXON_OK) return st;
@@ -208,6 +233,65 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
   return AXON_OK;
 }
 
+// The bit-plane form's memory: per network its activity words; per trajectory slot the records
+// of its spikes, the planes of its candidate columns, drives, thresholds, a row of the done
+// buffer and its part of the tick's tables.
+axon_status axon_server::start_planes(uint64_t memBytes) {
+  const uint32_t n = (uint32_t)nets.size(), ngrp = ncol / 8u, ncw = ncol / 32u;
+  const size_t actBytes = al(2ull * ngrp * (kServeMaxB / 32u) * 4);
+  const uint64_t fixed = n * actBytes + al(n * sizeof(PlanesTeam)) + al(n * 128) + al((size_t)n * kServeMaxB * 4) + 2048;
+  const size_t recB = (size_t)(ngrp + ncol) * 16, planeB = (size_t)ncol * 64, candB = (size_t)ncw * 4, drvB = (size_t)ncol * 4;
+  const size_t perSlot = recB + planeB + candB + drvB + 8 + (size_t)ncol * 4 + sizeof(PlanesEntry) + (size_t)incols * 4;
+  if (memBytes <= fixed + perSlot + 64) return set_error(AXON_EINVAL, "memory budget below one trajectory slot");
+  nslots = (uint32_t)std::min<uint64_t>((memBytes - fixed) / (perSlot + 64), 1u << 16);
+  slotCost = perSlot + 64;
+  fixedCost = fixed;
+  stageBytes = 1024 + al(n * sizeof(PlanesTeam)) + al(n * 128) + al(nslots * sizeof(PlanesEntry)) +
+               al((size_t)n * kServeMaxB * 4) + al((size_t)nslots * incols * 4);
+  size_t off = 0;
+  auto place = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
+  const size_t oErr = place(64), oAct = place(n * actBytes), oCand = place(nslots * candB), oTh = place(nslots * 8ull),
+               oRec = place(nslots * recB), oPlane = place(nslots * planeB), oDrv = place(nslots * drvB),
+               oStage = place(stageBytes), oDone = place((size_t)nslots * ncol * 4);
+  if (cudaMalloc(&dmem, off) != cudaSuccess) {
+    cudaGetLastError();
+    dmem = nullptr;
+    return set_error(AXON_ENOMEM, "server device allocation failed");
+  }
+  CKS(cudaMallocHost(&hmem, stageBytes));
+  CKS(cudaMallocHost(&hdone, (size_t)nslots * ncol * 4));
+  CKS(cudaMallocHost((void**)&herr, 64));
+  CKS(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  for (auto& evp : ev)
+    for (auto& e : evp) CKS(cudaEventCreate(&e));
+  char* b = (char*)dmem;
+  CKS(cudaMemsetAsync(b, 0, oRec, stream));  // error word, activity and candidate bits, thresholds
+  actMem = (uint32_t*)(b + oAct);
+  pdev.rec = (uint4*)(b + oRec);
+  pdev.candB = (uint32_t*)(b + oCand);
+  pdev.candP = (uint4*)(b + oPlane);
+  pdev.drv = (uint32_t*)(b + oDrv);
+  pdev.drvB = ncol;
+  pdev.drvC = 1u;
+  pdev.thPrev = (uint32_t*)(b + oTh);
+  pdev.thStride = nslots;
+  pdev.finalOut = (uint32_t*)(b + oDone);
+  pdev.err = (uint32_t*)(b + oErr);
+  dev.counts = (const uint32_t*)(b + oStage);
+  dev.doneBuf = pdev.finalOut;
+  dev.err = pdev.err;
+  pcfg.ncol = ncol; pcfg.incols = incols; pcfg.k = cfg.k; pcfg.dthr = cfg.dthr; pcfg.mode = cfg.mode;
+  pcfg.targetCols = cfg.targetCols; pcfg.topkPar = cfg.topkPar; pcfg.bst = cfg.bst; pcfg.waitNs = nets[0]->wait_ns;
+  CKS(planes_serve_prepare(pcfg));
+  CKS(cudaStreamSynchronize(stream));
+  for (uint32_t s = nslots; s-- > 0;) freeSlots.push_back(s);
+  act.assign(n, {});
+  netPar.assign(n, 0u);
+  laneUsed.assign(n, std::vector<uint32_t>(kServeMaxB / 32u, 0u));
+  th = std::thread([this] { loop(); });
+  return AXON_OK;
+}
+
 axon_server::~axon_server() {
   {
     std::lock_guard<std::mutex> g(mu);
@@ -245,29 +329,184 @@ void axon_server::loop() {
       }
     }
     const double t0 = now_s();
-    const axon_status s = tick();
+    const axon_status s = planes ? tick_planes() : tick();
     if (s != AXON_OK) { fail(s, axon_last_error()); return; }
     std::lock_guard<std::mutex> g(mu);
     busy += now_s() - t0;
   }
 }
 
-axon_status axon_server::tick() {
-  // admission: arrived requests, in arrival order, into free slots, while the request's
-  // network has room in its batch
+// admission: arrived requests, in arrival order, into free slots, while the request's network
+// has room in its batch
+void axon_server::admit() {
+  std::lock_guard<std::mutex> g(mu);
+  const double t = now_s();
+  while (!queue.empty() && !freeSlots.empty() && queue.front().arrive <= t && act[queue.front().net].size() < capB) {
+    Active a{freeSlots.back(), 0u, 0u, std::move(queue.front())};
+    freeSlots.pop_back();
+    queue.pop_front();
+    a.req.admit = t;
+    if (planes) {  // the lowest free lane
+      std::vector<uint32_t>& used = laneUsed[a.req.net];
+      uint32_t w = 0;
+      while (used[w] == 0xFFFFFFFFu) ++w;
+      const uint32_t bit = (uint32_t)__builtin_ctz(~used[w]);
+      used[w] |= 1u << bit;
+      a.lane = 32u * w + bit;
+    }
+    act[a.req.net].push_back(std::move(a));
+    ++nActive;
+    ++nRunning;
+  }
+}
+
+// One launch of the bit-plane form. Every trajectory takes the same number of steps: up to
+// kServeSteps, but no more than the one with the fewest left (so that none waits for the
+// launch's end), nor than fit before the next request known to arrive.
+axon_status axon_server::tick_planes() {
+  admit();
+  if (nRunning == 0) return retire_pending();
+  uint32_t steps = kServeSteps;
   {
     std::lock_guard<std::mutex> g(mu);
-    const double t = now_s();
-    while (!queue.empty() && !freeSlots.empty() && queue.front().arrive <= t && act[queue.front().net].size() < capB) {
-      Active a{freeSlots.back(), 0u, std::move(queue.front())};
-      freeSlots.pop_back();
-      queue.pop_front();
-      a.req.admit = t;
-      act[a.req.net].push_back(std::move(a));
-      ++nActive;
-      ++nRunning;
+    if (!queue.empty()) {
+      const double gap = queue.front().arrive - now_s();
+      if (gap > 0 && stepS > 0) steps = (uint32_t)std::min<double>(steps, 1.0 + gap / stepS);
     }
   }
+  uint32_t nact = 0, total = 0, maxB = 0, maxCols = 0;
+  for (const std::vector<Active>& A : act) {
+    for (const Active& a : A) steps = std::min(steps, a.req.steps - a.tloc);
+    nact += !A.empty();
+    total += (uint32_t)A.size();
+  }
+  teamH.clear();
+  pentH.clear();
+  laneH.clear();
+  cueH.clear();
+  // CTAs in proportion to a network's trajectories (plus a share for its tiles), one at least
+  uint32_t ndone = 0, cta = 0, left = nact, weightLeft = total + 16u * nact;
+  const uint32_t grid = (uint32_t)sms;
+  std::vector<size_t> laneOff;
+  bool wide = false;  // a team has more trajectories than CTAs
+  for (uint32_t n = 0; n < (uint32_t)act.size(); ++n) {
+    const std::vector<Active>& A = act[n];
+    if (A.empty()) continue;
+    const uint32_t weight = (uint32_t)A.size() + 16u, room = grid - cta - (left - 1u);
+    const uint32_t ncta = left == 1u ? grid - cta
+                                     : std::max(1u, std::min(room, (uint32_t)((uint64_t)(grid - cta) * weight / weightLeft)));
+    PlanesTeam T{};
+    T.net.W3P = nets[n]->w3p;
+    T.net.conn = nets[n]->d.conn;
+    T.net.act = actMem + (size_t)n * (al(2ull * (ncol / 8u) * (kServeMaxB / 32u) * 4) / 4);
+    T.net.astr = kServeMaxB / 32u;
+    T.net.par = netPar[n];
+    T.cta0 = cta;
+    T.ncta = ncta;
+    for (const Active& a : A) T.B = std::max(T.B, a.lane + 1u);
+    maxB = std::max(maxB, T.B);
+    maxCols = std::max(maxCols, (ncol + ncta - 1u) / ncta);
+    wide = wide || T.B > ncta;
+    laneOff.push_back(laneH.size());
+    laneH.resize(laneH.size() + T.B, kNoSlot);
+    for (const Active& a : A) {
+      PlanesEntry e{};
+      e.slot = a.slot;
+      e.t0 = a.tloc;
+      e.clamp = a.req.clamp;
+      e.steps = a.req.steps;
+      if (a.tloc < a.req.clamp) {
+        e.ncue = (uint32_t)a.req.cue.size();
+        e.cueOff = (uint32_t)cueH.size();
+        cueH.insert(cueH.end(), a.req.cue.begin(), a.req.cue.end());
+      }
+      e.done = a.tloc + steps == a.req.steps ? ndone++ : kNoSlot;
+      laneH[laneOff.back() + a.lane] = (uint32_t)pentH.size();
+      pentH.push_back(e);
+    }
+    netPar[n] ^= steps & 1u;
+    cta += ncta;
+    --left;
+    weightLeft -= weight;
+    teamH.push_back(T);
+  }
+  // one upload: [teams][their barriers, zero][entries][lanes][cues]
+  const uint32_t nt = (uint32_t)teamH.size(), ne = (uint32_t)pentH.size();
+  const size_t oBar = al(nt * sizeof(PlanesTeam)), oEnt = oBar + al(nt * 128), oLane = oEnt + al(ne * sizeof(PlanesEntry)),
+               oCue = oLane + al(laneH.size() * 4), bytes = oCue + cueH.size() * 4;
+  char* h = (char*)hmem;
+  char* ds = (char*)dev.counts;
+  for (uint32_t i = 0; i < nt; ++i) {
+    teamH[i].net.bar = (uint32_t*)(ds + oBar + 128u * i);
+    teamH[i].net.lanes = (const uint32_t*)(ds + oLane) + laneOff[i];
+  }
+  std::memcpy(h, teamH.data(), nt * sizeof(PlanesTeam));
+  std::memset(h + oBar, 0, nt * 128);
+  std::memcpy(h + oEnt, pentH.data(), ne * sizeof(PlanesEntry));
+  std::memcpy(h + oLane, laneH.data(), laneH.size() * 4);
+  if (!cueH.empty()) std::memcpy(h + oCue, cueH.data(), cueH.size() * 4);
+  PlanesDev td = pdev;
+  td.teams = (const PlanesTeam*)ds;
+  td.nteams = nt;
+  td.entries = (const PlanesEntry*)(ds + oEnt);
+  td.cues = (const uint32_t*)(ds + oCue);
+  PlanesCfg tc = pcfg;
+  tc.B = maxB;
+  tc.T = steps;
+  const PlanesShape sh = planes_serve_shape(ncol, maxB, (int)cta, maxCols, wide ? 3u : 1u, &tc);
+  const double t0 = now_s();
+  CKS(cudaMemcpyAsync(ds, h, bytes, cudaMemcpyHostToDevice, stream));
+  const uint32_t eb = pendingEv ^ 1u;  // this launch's events (the previous one's are still to be read)
+  CKS(cudaEventRecord(ev[eb][0], stream));
+  CKS(launch_serve_planes(td, tc, sh, stream));
+  CKS(cudaEventRecord(ev[eb][1], stream));
+  CKS(cudaEventRecord(ev[eb][2], stream));
+  {  // while the GPU runs: the previous launch's results
+    const axon_status st = retire_pending();
+    if (st != AXON_OK) return st;
+  }
+  if (ndone) CKS(cudaMemcpyAsync(hdone, dev.doneBuf, (size_t)ndone * ncol * 4, cudaMemcpyDeviceToHost, stream));
+  CKS(cudaMemcpyAsync(herr, dev.err, 4, cudaMemcpyDeviceToHost, stream));
+  pending.clear();
+  uint32_t ei = 0;
+  for (uint32_t n = 0; n < (uint32_t)act.size(); ++n) {
+    std::vector<Active>& A = act[n];
+    size_t w = 0;
+    for (size_t i = 0; i < A.size(); ++i) {
+      Active& a = A[i];
+      const PlanesEntry& e = pentH[ei++];
+      if (e.done != kNoSlot) {
+        Finished f{};
+        f.r.tag = a.req.tag;
+        f.r.net = a.req.net;
+        f.r.steps = a.req.steps;
+        f.r.arrive_s = a.req.arrive;
+        f.r.admit_s = a.req.admit;
+        f.done = e.done;
+        f.slot = a.slot;
+        pending.push_back(f);
+        laneUsed[n][a.lane >> 5] &= ~(1u << (a.lane & 31u));
+      } else {
+        a.tloc += steps;
+        if (w != i) A[w] = std::move(a);
+        ++w;
+      }
+    }
+    A.resize(w);
+  }
+  nRunning -= pending.size();
+  pendingTick = true;
+  pendingNe = ne;
+  pendingSteps = steps;
+  pendingEv = eb;
+  CKS(cudaStreamSynchronize(stream));
+  stepS = (now_s() - t0) / steps;
+  if (herr[0] != 0u) return set_error(AXON_ETIMEOUT, "a wait timed out in the serving kernel");
+  return AXON_OK;
+}
+
+axon_status axon_server::tick() {
+  admit();
   if (nRunning == 0) return retire_pending();
   // the tick's tables: every network's trajectories in batch-index order; a network with
   // many of them is advanced by the batched kernel, the others by the gather kernel
@@ -415,10 +654,10 @@ axon_status axon_server::retire_pending() {
   for (auto& d : fin) done.push_back(std::move(d));
   for (const Finished& f : pending) freeSlots.push_back(f.slot);
   nActive -= pending.size();
-  ++ticks;
+  ticks += pendingSteps;
   driveS += msDrive * 1e-3;
   emitS += msEmit * 1e-3;
-  sumActive += pendingNe;
+  sumActive += (uint64_t)pendingNe * pendingSteps;
   maxActive = std::max<uint64_t>(maxActive, pendingNe);
   completed += pending.size();
   pending.clear();

@@ -338,7 +338,7 @@ typedef struct axon_serve_counters {
   uint64_t max_batch;  /* most trajectories advanced in one tick */
   double mean_batch;   /* trajectories per tick, mean */
   double busy_s;       /* time spent in ticks */
-  double drive_s;      /* device time of the drive kernel, summed over ticks */
+  double drive_s;      /* device time of the drive kernel, summed over ticks (of the whole step when one kernel runs it) */
   double emit_s;       /* device time of the threshold/emit kernel, summed over ticks */
   uint64_t slot_bytes; /* device memory one trajectory slot takes */
   uint64_t fixed_bytes;/* device memory of the server besides its slots: slots = (mem_bytes - fixed) / slot */
