@@ -55,7 +55,7 @@ PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c) {
   // columns are staged (us per step, read / staged: 33 / 70 at 32 trajectories, 50 / 70 at 64,
   // 64 / 76 at 112, 73 / 79 at 150, 81 / 82 at 176)
   s.direct = B <= kPlanesDirectB ? 1u : 0u;
-  s.smem = planes_fit(ncol, B, s.direct != 0u, (ncol + (uint32_t)sms - 1u) / (uint32_t)sms, (B + (uint32_t)sms - 1u) / (uint32_t)sms,
+  s.smem = planes_fit(ncol, B, s.direct != 0u, false, (ncol + (uint32_t)sms - 1u) / (uint32_t)sms, (B + (uint32_t)sms - 1u) / (uint32_t)sms,
                       c);
   return s;
 }

@@ -12,12 +12,14 @@ namespace axon {
 // i = the neurons whose number of functional synapses in the word has bit i set); then two
 // zero words, which padding entries of a record's position list point at.
 constexpr uint32_t kPlaneBlk = 40;
-constexpr uint32_t kPlaneTile = 8u * kPlaneBlk;     // one (column, branch)
+// one (column, branch): the eight blocks and four words more, so that the row-count planes of
+// different branches and words spread over all shared-memory banks
+constexpr uint32_t kPlaneTile = 8u * kPlaneBlk + 4u;
 constexpr uint32_t kPlaneCol = 32u * kPlaneTile;    // one column
 constexpr uint32_t kPlanes = 14;                    // bit planes of a per-neuron drive (below 2^14)
 constexpr uint32_t kPlanesMaxB = 512;               // trajectories per launch (the host splits larger batches)
-constexpr uint32_t kPlanesVals = 1536;              // candidates a phase-2 group keeps in shared memory
-constexpr uint32_t kPlanesList = 512;               // gated columns it lists there
+constexpr uint32_t kPlanesVals = 1024;              // candidates a phase-2 group keeps in shared memory
+constexpr uint32_t kPlanesList = 384;               // gated columns it lists there
 // 640 threads leave 96 registers; tiles read through L2 want more warps (at most 28: a phase-2
 // group keeps two words per warp beside its counters)
 constexpr int planes_threads(bool direct) { return direct ? 896 : 640; }
@@ -59,6 +61,7 @@ struct PlanesDev {
   uint32_t* candB;          // [B][ncol/32] candidates of the step, a bit per column (zeroed before the launch)
   uint4* candP;             // [B][ncol][4] their drive planes (words 0..13); word 15: the ballot, in a step with more
                             // than kPlanesList gated columns
+  uint4* aff;               // [ncol][32 * blocks][4] planes of the input groups' share of the drives, or null
   uint32_t* drv;            // column drives of the step, trajectory b's column c at b * drvB + c * drvC
   uint32_t* thPrev;         // [2][thStride] the last two thresholds, by step parity
   uint32_t* finalOut;       // [B][ncol] spikes of the last step (zeroed before the launch), or null
@@ -82,6 +85,7 @@ struct PlanesCfg {
   uint32_t ns, nl, ng;   // tile slots, list slots (0 when direct), phase-2 groups
   uint32_t nsl, nll;     // log2 of ns and nl
   uint32_t ls;           // log2 of the lanes per trajectory in phase 1
+  uint32_t aff;          // 1: the afferent cache pays
   uint64_t waitNs;
 };
 

@@ -39,8 +39,8 @@
 // atomics. 640 threads leave 96 registers a thread (896 threads spilled and took 8 % longer).
 // The L2 form has 896 threads: it waits for its reads, not for the pipes.
 // Measured per step, config C at load 60 (batch.cu / this): 69 / 16 us for one trajectory,
-// 86 / 24 for 16, 96 / 50 for 64, 98 / 59 for 100, 111 / 84 for 200, 133 / 106 for 300, 213 /
-// 168 for 512.
+// 86 / 24 for 16, 96 / 47 for 64, 98 / 56 for 100, 111 / 78 for 200, 133 / 101 for 300, 213 /
+// 162 for 512.
 #pragma once
 #include <cstdint>
 
@@ -319,11 +319,9 @@ __device__ __forceinline__ void accumulate(Tile tile, Tile conn, uint32_t m, uin
   } while (!last);
 }
 
-// Per-neuron drive planes from the sums: D (in A) = A + bst * M (modes 0, 1) or M (mode 2),
-// minus the bias (saturating at zero).
+// Per-neuron drive planes from the sums: D (in A) = A + bst * M (modes 0, 1) or M (mode 2).
 template <bool LIN>
-__device__ __forceinline__ void finish_planes(uint32_t (&A)[kPlanes], const uint32_t (&M)[6], uint32_t bst,
-                                              const uint32_t* biasP) {
+__device__ __forceinline__ void combine_planes(uint32_t (&A)[kPlanes], const uint32_t (&M)[6], uint32_t bst) {
   if (LIN) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -338,17 +336,28 @@ __device__ __forceinline__ void finish_planes(uint32_t (&A)[kPlanes], const uint
 #pragma unroll
     for (int i = 0; i < 6; ++i) A[i] = M[i];
   }
-  if (biasP) {
-    uint32_t b = 0u;
+}
+
+// D + the drive planes at p
+__device__ __forceinline__ void add_planes(uint32_t (&D)[kPlanes], const uint4* p) {
+  const uint4 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(p + 2), e = __ldcg(p + 3);
+  const uint32_t P[kPlanes] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w, e.x, e.y};
+  uint32_t k = 0u;
 #pragma unroll
-    for (int i = 0; i < (int)kPlanes; ++i) {
-      const uint32_t p = __ldg(biasP + i), x = A[i];
-      A[i] = x ^ p ^ b;
-      b = (~x & (p | b)) | (p & b);
-    }
+  for (int i = 0; i < (int)kPlanes; ++i) fa(D[i], P[i], k, D[i], k);
+}
+
+// D minus the bias, saturating at zero
+__device__ __forceinline__ void subtract_bias(uint32_t (&D)[kPlanes], const uint32_t* biasP) {
+  uint32_t b = 0u;
 #pragma unroll
-    for (int i = 0; i < (int)kPlanes; ++i) A[i] &= ~b;
+  for (int i = 0; i < (int)kPlanes; ++i) {
+    const uint32_t p = __ldg(biasP + i), x = D[i];
+    D[i] = x ^ p ^ b;
+    b = (~x & (p | b)) | (p & b);
   }
+#pragma unroll
+  for (int i = 0; i < (int)kPlanes; ++i) D[i] &= ~b;
 }
 
 // sum over the neurons in `mask` of the drives held in planes D
@@ -521,7 +530,8 @@ __device__ __noinline__ void recompute_planes(const PlanesNet& net, const Planes
   accumulate<GlobalTile, LIN, DT1>(GlobalTile{reinterpret_cast<const char*>(net.W3P + (size_t)col * kPlaneCol)},
                                    GlobalTile{reinterpret_cast<const char*>(net.conn + col * kNslot)}, m, 0u, rec, ngrp,
                                    c.dthr, D, M);
-  finish_planes<LIN>(D, M, c.bst, biasP);
+  combine_planes<LIN>(D, M, c.bst);
+  if (biasP) subtract_bias(D, biasP);
   store_planes(p, D);
 }
 
@@ -533,8 +543,8 @@ __host__ __device__ inline uint32_t group_words(uint32_t ncol) {
 __host__ __device__ inline uint32_t list_words(uint32_t nblk) { return 48u * nblk + 36u; }
 constexpr uint32_t kMaxNS = 4, kMaxNL = 8;  // tile and list slots
 // phase 1's tables: activity words, floors, state slots, lists
-__host__ __device__ inline uint32_t table_words(uint32_t ncol, uint32_t nblk, uint32_t nl) {
-  return ncol / 8u * nblk + 64u * nblk + nl * list_words(nblk);
+__host__ __device__ inline uint32_t table_words(uint32_t ncol, uint32_t nblk, uint32_t nl, bool serve) {
+  return ncol / 8u * nblk + (serve ? 64u : 32u) * nblk + nl * list_words(nblk);
 }
 constexpr uint32_t kCtlWords = 2u * (kMaxNS + 2u * kMaxNL) + 4u + 2u * kMaxNS + 2u * kMaxNL;
 
@@ -573,7 +583,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
                                         // them: from global memory a few L2 lines would serve them all)
   uint32_t* sFloor = sAct + ngrp * nblk;  // [Bp] candidate floors
   uint32_t* sSlot = sFloor + Bp;          // [Bp] SERVE: state slots (kNoSlot: none, or at its end)
-  uint32_t* sLists = sSlot + Bp;          // [c.nl][list_words]
+  uint32_t* sLists = sSlot + (SERVE ? Bp : 0u);  // [c.nl][list_words]
   uint32_t* sGrp = sAct;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = blockDim.x >> 5;
   const uint32_t ncols = cta < ncol ? (ncol - cta + G - 1u) / G : 0u;  // columns cta, cta + G, ...
@@ -606,19 +616,30 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
   // and lists the trajectories for a column: each one's active branches (the activity words of
   // the column's 32 groups, transposed), the trajectories by falling number of them, so that
   // the 32 lanes of a task have nearly equal work
-  auto list = [&](uint32_t slot, uint32_t ci) {
+  auto conn_row = [&](uint32_t ci) { return __ldg(net.conn + (cta + ci * G) * kNslot + lane); };
+  auto list = [&](uint32_t slot, uint32_t g, uint32_t skip) {
     uint32_t* sM = sLists + slot * list_words(nblk);
     uint16_t* sOrd = reinterpret_cast<uint16_t*>(sM + Bp);
     uint32_t* sCount = sM + 48u * nblk;  // [33]
-    const uint32_t* row = sAct + __ldg(net.conn + (cta + ci * G) * kNslot + lane) * nblk;
+    const uint32_t* row = sAct + g * nblk;
     sCount[lane] = 0u;
     if (lane == 0) sCount[32] = 0u;
     __syncwarp();
-#pragma unroll 2
-    for (uint32_t k = 0; k < nblk; ++k) {
-      const uint32_t m = transpose32(row[k], lane);
-      sM[32u * k + lane] = m;
-      atomicAdd(sCount + __popc(m), 1u);
+    // several blocks at a time, their loads, transposes and stores in groups: taken one by one
+    // (the stores keep the next block's load behind them) a list of ten blocks took 4 us
+    constexpr uint32_t kU = DIRECT ? 2 : 5;
+    for (uint32_t k0 = 0; k0 < nblk; k0 += kU) {
+      uint32_t m[kU];
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i) m[i] = k0 + i < nblk && g >= skip ? row[k0 + i] : 0u;
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i) m[i] = transpose32(m[i], lane);
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i)
+        if (k0 + i < nblk) {
+          sM[32u * (k0 + i) + lane] = m[i];
+          atomicAdd(sCount + __popc(m[i]), 1u);
+        }
     }
     __syncwarp();
     const uint32_t n = sCount[32u - lane];
@@ -632,8 +653,17 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
     sCount[32u - lane] = at - n;
     if (lane == 31u) sCount[0] = at;
     __syncwarp();
-#pragma unroll 2
-    for (uint32_t b = lane; b < Bp; b += 32u) sOrd[atomicAdd(sCount + __popc(sM[b]), 1u)] = (uint16_t)b;
+    for (uint32_t k0 = 0; k0 < nblk; k0 += kU) {
+      uint32_t o[kU];
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i) o[i] = k0 + i < nblk ? (uint32_t)__popc(sM[32u * (k0 + i) + lane]) : 33u;
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i)
+        if (k0 + i < nblk) o[i] = atomicAdd(sCount + o[i], 1u);
+#pragma unroll
+      for (uint32_t i = 0; i < kU; ++i)
+        if (k0 + i < nblk) sOrd[o[i]] = (uint16_t)(32u * (k0 + i) + lane);
+    }
     __syncwarp();
     if (!DIRECT && lane == 0) {
       sMade[slot] += 1u;
@@ -658,8 +688,18 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
     const uint32_t ap = (t + net.par) & 1u;
     const uint32_t* actIn = net.act + (size_t)ap * ngrp * net.astr;
     uint32_t* actOut = net.act + (size_t)(ap ^ 1u) * ngrp * net.astr;
+    // Afferent cache. While the inputs are clamped their spikes are the cue at every step, so
+    // the input groups' share of the drives is the same in steps 1..clampSteps. Step 1, whose
+    // drives are that share alone (no recurrent column spikes at step 0), stores its planes;
+    // the others leave the input groups out, half of the clamped steps' spike words, and add
+    // the stored planes.
+    const bool affStore = !SERVE && d.aff != nullptr && t == 1u;
+    const bool affAdd = !SERVE && d.aff != nullptr && t >= 2u && t <= c.clampSteps;
+    const uint32_t skip = affAdd ? incols / 8u : 0u;  // the groups below are left out
     // ---------------- phase 1 (nothing spikes before step 0: every drive is zero there)
     if (SERVE || t > 0u || d.refBall != nullptr) {
+      uint32_t g0 = 0;  // the connection row of the warp's first list, on its way during the copies below
+      if (!DIRECT && warp < NL && warp < ncols) g0 = conn_row(back ? ncols - 1u - warp : warp);
       if (SERVE) {
         for (uint32_t g = tid; g < ngrp; g += blockDim.x)
           for (uint32_t k = 0; k < nblk; ++k) sAct[g * nblk + k] = __ldcg(actIn + g * net.astr + k);
@@ -683,9 +723,9 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
           sFloor[b] = b < B ? cand_floor(d.thPrev, d.thStride, b, t, c.clampSteps, c) : 0xFFFFFFFFu;
       }
       __syncthreads();
-      if (!DIRECT && warp < NL && warp < ncols) list(warp, back ? ncols - 1u - warp : warp);
+      if (!DIRECT && warp < NL && warp < ncols) list(warp, g0, skip);
       if (DIRECT && sorted) {  // every column's list at once
-        for (uint32_t ci = warp; ci < ncols; ci += nw) list(ci, ci);
+        for (uint32_t ci = warp; ci < ncols; ci += nw) list(ci, conn_row(ci), skip);
         __syncthreads();
       }
       // the next step's activity words, last read in step t-1
@@ -704,7 +744,8 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
           m = sM[b];
         } else if (DIRECT) {
           b = at;
-          m = transpose32(sAct[__ldg(net.conn + col * kNslot + lane) * nblk + (b >> 5)], lane);
+          const uint32_t g = __ldg(net.conn + col * kNslot + lane);
+          m = transpose32(g >= skip ? sAct[g * nblk + (b >> 5)] : 0u, lane);
           if (ls) m = __shfl_sync(kFull, m, b & 31u);
         } else {
           const uint32_t u = q >> nsl, lu = q >> nll;
@@ -747,7 +788,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
                                            SharedTile{smem_u32(sConn + slot * 32u)}, m, ls, recb, ngrp, c.dthr, A,
                                            M);
         __syncwarp();
-        uint32_t last = 0;
+        uint32_t last = 0, gl = 0;
         if (!DIRECT) {  // the warp that finishes a column's last task refills its slots
           if (lane == 0) {
             mbar_arrive(&sBarE[lslot]);
@@ -755,6 +796,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
             if (last) mbar_wait(&sBarE[lslot], ln & 1u, c.waitNs);  // every arrival is made: orders the others' reads
           }
           last = __shfl_sync(kFull, last, 0);
+          if (last && q + NL < ncols) gl = conn_row(back ? ncols - 1u - (q + NL) : q + NL);
           if (last && q + NS < ncols) fill(slot, back ? ncols - 1u - (q + NS) : q + NS);
         }
         for (uint32_t o = 1; o < (1u << ls); o <<= 1) {  // the sums of a trajectory's lanes
@@ -767,7 +809,12 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
 #pragma unroll
           for (int i = 0; i < 6; ++i) fa(M[i], __shfl_xor_sync(kFull, M[i], o), k2, M[i], k2);
         }
-        finish_planes<LIN>(A, M, c.bst, d.biasP ? d.biasP + col * 16u : nullptr);
+        combine_planes<LIN>(A, M, c.bst);
+        if (!SERVE && part == 0u && b < B) {
+          if (affStore) store_planes(d.aff + ((size_t)col * Bp + b) * 4u, A);
+          if (affAdd) add_planes(A, d.aff + ((size_t)col * Bp + b) * 4u);
+        }
+        if (!SERVE && d.biasP) subtract_bias(A, d.biasP + col * 16u);
         const uint32_t s = plane_sum(A, kFull);
         if (part == 0u && (SERVE ? sl != kNoSlot : b < B)) {
           __stcg(d.drv + (size_t)sl * d.drvB + (size_t)col * d.drvC, s);
@@ -786,7 +833,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
         if (last) {
           __syncwarp();
           if (lane == 0) sDone[lslot] = 0u;
-          if (q + NL < ncols) list(lslot, back ? ncols - 1u - (q + NL) : q + NL);
+          if (q + NL < ncols) list(lslot, gl, skip);
         }
       }
       __syncthreads();
@@ -977,8 +1024,8 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
 
 
 namespace {
-size_t planes_smem(uint32_t ncol, uint32_t B, uint32_t ns, uint32_t nl, uint32_t ng) {
-  const size_t table = table_words(ncol, (B + 31u) / 32u, nl), groups = (size_t)ng * group_words(ncol);
+size_t planes_smem(uint32_t ncol, uint32_t B, uint32_t ns, uint32_t nl, uint32_t ng, bool serve) {
+  const size_t table = table_words(ncol, (B + 31u) / 32u, nl, serve), groups = (size_t)ng * group_words(ncol);
   return ((size_t)ns * (kPlaneCol + 32u) + kCtlWords + (table > groups ? table : groups)) * 4u;
 }
 template <bool LIN, bool DT1, bool SERVE>
@@ -993,7 +1040,7 @@ const void* planes_fn(const PlanesCfg& c, uint32_t direct) {
 
 // Shared-memory shares for at most B trajectories in one team, `cols` columns in one CTA and
 // `want` phase-2 groups.
-size_t planes_fit(uint32_t ncol, uint32_t B, bool direct, uint32_t cols, uint32_t want, PlanesCfg* c) {
+size_t planes_fit(uint32_t ncol, uint32_t B, bool direct, bool serve, uint32_t cols, uint32_t want, PlanesCfg* c) {
   constexpr size_t kLimit = 227u * 1024u;
   // lanes per trajectory: one, but a handful of trajectories would leave most lanes idle while
   // the others walk eight branches in a row (us per step at 1 / 8 / 16 / 24 trajectories of a
@@ -1004,20 +1051,34 @@ size_t planes_fit(uint32_t ncol, uint32_t B, bool direct, uint32_t cols, uint32_
   c->nsl = 2;
   c->nll = 3;
   c->ng = want < 3u ? want : 3u;
-  auto fits = [&]() { return planes_smem(ncol, B, c->ns, c->nl, c->ng) <= kLimit; };
+  auto bytes = [&]() { return planes_smem(ncol, B, c->ns, c->nl, c->ng, serve); };
+  auto fits = [&]() { return bytes() <= kLimit; };
   if (!direct) {
+    // within 195 KiB, where that is possible with four list slots, the L1 has 60 KiB instead of
+    // 28, which the record gathers feel (us per step, 28 / 60 KiB: 107 / 101 at 300
+    // trajectories, 111 / 102 at 320)
+    constexpr size_t kRoomy = 195u * 1024u;
     c->ns = 1u << c->nsl;
     c->nl = 1u << c->nll;
+    if (bytes() > kRoomy) {
+      c->nl = 4u;
+      if (bytes() <= kRoomy) c->nll = 2u;
+      else c->nl = 1u << c->nll;
+    }
     while (c->ng > 2u && !fits()) --c->ng;
     if (!fits()) { c->nsl = 1; c->ns = 2; }
     if (!fits()) { c->nll = 2; c->nl = 4; }
   }
   while (c->ng > 1u && !fits()) --c->ng;
+  // with the small L1 the afferent cache's reads cost more than they save (us per step,
+  // without / with it: 74 / 70 at 160, 89 / 86 at 256, 104 / 101 at 300; but 115 / 119 at 352
+  // and 163 / 170 at 512)
+  c->aff = direct || bytes() <= 195u * 1024u ? 1u : 0u;
   if (direct && B > 32u) {  // a list for each of a CTA's columns, where that leaves the L1 most of its memory
     c->nl = cols;
     if (c->nl * list_words((B + 31u) / 32u) * 4u > 64u * 1024u || !fits()) c->nl = 0;
   }
-  return planes_smem(ncol, B, c->ns, c->nl, c->ng);
+  return bytes();
 }
 }  // namespace
 

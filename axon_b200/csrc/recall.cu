@@ -87,7 +87,17 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   const size_t zBytes = al(2ull * ngrp * nblk * 4) + al((size_t)Bc * (ncol / 32u) * 4) + al((size_t)Bc * 8) + 256;
   const size_t need = zBytes + al((size_t)Bc * (ngrp + ncol) * 16) + al((size_t)ncol * nblk * 32 * 4) + al(bnc * 64) +
                       al((size_t)ncol * 64) + al((size_t)ncol * 4);
-  axon_status st = scratch.ensure(need);
+  // the afferent cache, when steps 2.. are clamped and the input columns fill whole groups (a
+  // group of input and recurrent columns changes while clamped); without it where it does not
+  // fit the memory that is left
+  planes_shape(ncol, Bc, sm_count, &c);
+  const size_t affBytes = c.aff && a.clamp_steps >= 2u && a.T >= 3u && cfg.incols % 8u == 0u ? al((size_t)ncol * nblk * 32 * 64) : 0;
+  bool useAff = affBytes != 0;
+  axon_status st = scratch.ensure(need + affBytes);
+  if (st != AXON_OK && useAff) {
+    useAff = false;
+    st = scratch.ensure(need);
+  }
   if (st != AXON_OK) return st;
   char* p = (char*)scratch.p;
   auto take = [&](size_t bytes) { char* r = p; p += al(bytes); return r; };
@@ -100,6 +110,7 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   d0.rec = (uint4*)take((size_t)Bc * (ngrp + ncol) * 16);
   d0.drv = (uint32_t*)take((size_t)ncol * nblk * 32 * 4);
   d0.candP = (uint4*)take(bnc * 64);
+  d0.aff = useAff ? (uint4*)take(affBytes) : nullptr;
   uint32_t* biasP = (uint32_t*)take((size_t)ncol * 64);
   uint32_t* multM = (uint32_t*)take((size_t)ncol * 4);
   d0.net.W3P = w3p;

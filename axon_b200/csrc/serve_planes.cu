@@ -11,7 +11,7 @@ PlanesShape planes_serve_shape(uint32_t ncol, uint32_t B, int grid, uint32_t col
   PlanesShape s{};
   s.grid = grid;
   s.direct = B <= kPlanesDirectB ? 1u : 0u;
-  s.smem = planes_fit(ncol, B, s.direct != 0u, cols, want, c);
+  s.smem = planes_fit(ncol, B, s.direct != 0u, true, cols, want, c);
   return s;
 }
 

@@ -84,3 +84,12 @@ def test_wide_networks_with_logs():
         for slab in ("floor", "floor_always", "full"):
             same(net, cues_of(net, pats, B, 3), 9, 3, ref_ball=ref if slab == "floor" else None, slab=slab)
         net.close()
+
+
+# the input groups' share of the drives, kept over the clamped steps: none, one, all but the last, all
+@pytest.mark.parametrize("clamp", [0, 1, 2, 7, 8, 9])
+@pytest.mark.parametrize("B", [13, 161, 300])
+def test_clamped_steps(clamp, B):
+    net, pats = trained(incols=72)
+    same(net, cues_of(net, pats, B, clamp), 8, clamp)
+    net.close()
