@@ -41,13 +41,14 @@ struct PlanesNet {
 struct PlanesTeam {
   PlanesNet net;
   uint32_t cta0, ncta, B;
+  uint32_t moved;  // lanes differ from those of the launch before: the first step's activity words are permuted
 };
 struct PlanesEntry {
   uint32_t slot;             // state slot
   uint32_t t0, clamp, steps;  // its step at the launch's first, clamped steps, all steps
   uint32_t ncue, cueOff;     // clamped input columns, in the launch's cue area
   uint32_t done;             // row of its final spikes when it ends in this launch
-  uint32_t pad;
+  uint32_t from;             // its lane in the launch before (a new trajectory's: one that no other has)
 };
 
 struct PlanesDev {

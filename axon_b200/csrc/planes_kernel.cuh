@@ -601,6 +601,12 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
   for (uint32_t i = tid; i < 4u + 2u * kMaxNS + 2u * kMaxNL; i += blockDim.x) sMisc[i] = 0u;
   __syncthreads();
 
+  const bool moved = SERVE && d.teams[team].moved != 0u;
+  auto lane_before = [&](uint32_t b) -> uint32_t {
+    const uint32_t ei = b < B ? __ldg(net.lanes + b) : kNoSlot;
+    return ei != kNoSlot ? d.entries[ei].from : kNoSlot;
+  };
+
   // a warp brings column ci of the CTA into a tile slot: the connection row by its lanes, the tiles by one bulk copy
   auto fill = [&](uint32_t slot, uint32_t ci) {
     const uint32_t col = cta + ci * G;
@@ -700,9 +706,29 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
     if (SERVE || t > 0u || d.refBall != nullptr) {
       uint32_t g0 = 0;  // the connection row of the warp's first list, on its way during the copies below
       if (!DIRECT && warp < NL && warp < ncols) g0 = conn_row(back ? ncols - 1u - warp : warp);
-      if (SERVE) {
+      if (SERVE && moved && t == 0u) {
+        // the trajectories have other lanes than in the launch before: a warp takes a group's
+        // old words, one per lane, and puts the new ones together bit by bit (about 3 us for
+        // 512 groups)
+        for (uint32_t b = tid; b < Bp; b += blockDim.x) sFloor[b] = lane_before(b);
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t g = warp; g < ngrp; g += nw) {
+          const uint32_t old = lane < net.astr ? __ldcg(actIn + g * net.astr + lane) : 0u;
+          uint32_t mine = 0u;
+          for (uint32_t k = 0; k < nblk; ++k) {
+            const uint32_t f = sFloor[32u * k + lane], w = __shfl_sync(kFull, old, (f >> 5) & 31u);
+            const uint32_t now = __ballot_sync(kFull, f != kNoSlot && ((w >> (f & 31u)) & 1u) != 0u);
+            if (lane == k) mine = now;
+          }
+          if (lane < nblk) sAct[g * nblk + lane] = mine;
+        }
+        __syncthreads();
+      } else if (SERVE) {
         for (uint32_t g = tid; g < ngrp; g += blockDim.x)
           for (uint32_t k = 0; k < nblk; ++k) sAct[g * nblk + k] = __ldcg(actIn + g * net.astr + k);
+      }
+      if (SERVE) {
         for (uint32_t b = tid; b < Bp; b += blockDim.x) {
           const uint32_t ei = b < B ? __ldg(net.lanes + b) : kNoSlot;
           uint32_t slot = kNoSlot, fl = 0xFFFFFFFFu;
@@ -989,7 +1015,8 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
         for (uint32_t i = grp.t; i < walk; i += grp.nt) {
           const uint32_t e = over ? i : sList[i];  // = the column
           if (over && !gated(val(e))) continue;
-          recompute_planes<LIN, DT1>(net, c, actIn, b, e, recb, d.biasP ? d.biasP + e * 16u : nullptr, candb + (size_t)e * 4u);
+          const uint32_t bit = SERVE && moved && t == 0u ? lane_before(b) : b;  // its place in the activity words
+          recompute_planes<LIN, DT1>(net, c, actIn, bit, e, recb, d.biasP ? d.biasP + e * 16u : nullptr, candb + (size_t)e * 4u);
         }
       for (uint32_t i = grp.t; i < walk; i += grp.nt) {
         const uint32_t e = over ? i : sList[i];
@@ -1074,9 +1101,11 @@ size_t planes_fit(uint32_t ncol, uint32_t B, bool direct, bool serve, uint32_t c
   // without / with it: 74 / 70 at 160, 89 / 86 at 256, 104 / 101 at 300; but 115 / 119 at 352
   // and 163 / 170 at 512)
   c->aff = direct || bytes() <= 195u * 1024u ? 1u : 0u;
-  if (direct && B > 32u) {  // a list for each of a CTA's columns, where that leaves the L1 most of its memory
+  // a list for each of a CTA's columns, within 160 KiB (four teams of 4,096 columns, us per step
+  // without / with 122 to 147 KiB of lists: 293 / 265 at 160 trajectories in the largest, 240 / 209 at 127)
+  if (direct && B > 32u) {
     c->nl = cols;
-    if (c->nl * list_words((B + 31u) / 32u) * 4u > 64u * 1024u || !fits()) c->nl = 0;
+    if (c->nl * list_words((B + 31u) / 32u) * 4u > 160u * 1024u || !fits()) c->nl = 0;
   }
   return bytes();
 }

@@ -390,7 +390,7 @@ axon_status axon_server::tick_planes() {
   std::vector<size_t> laneOff;
   bool wide = false;  // a team has more trajectories than CTAs
   for (uint32_t n = 0; n < (uint32_t)act.size(); ++n) {
-    const std::vector<Active>& A = act[n];
+    std::vector<Active>& A = act[n];
     if (A.empty()) continue;
     const uint32_t weight = (uint32_t)A.size() + 16u, room = grid - cta - (left - 1u);
     const uint32_t ncta = left == 1u ? grid - cta
@@ -404,13 +404,25 @@ axon_status axon_server::tick_planes() {
     T.cta0 = cta;
     T.ncta = ncta;
     for (const Active& a : A) T.B = std::max(T.B, a.lane + 1u);
+    // A network's trajectories move to its lowest lanes when that saves a block of 32, or half
+    // of a small batch: a launch takes as long as its highest lane asks for (of a burst of
+    // 1,200 requests, four networks' last 128 in lanes up to 303 took 368 us per step,
+    // and 106 moved together).
+    T.moved = (T.B + 31u) / 32u > ((uint32_t)A.size() + 31u) / 32u || T.B >= 2u * (uint32_t)A.size();
+    if (T.moved) {
+      T.B = (uint32_t)A.size();
+      laneUsed[n].assign(laneUsed[n].size(), 0u);
+      for (uint32_t b = 0; b < T.B; ++b) laneUsed[n][b >> 5] |= 1u << (b & 31u);
+    }
     maxB = std::max(maxB, T.B);
     maxCols = std::max(maxCols, (ncol + ncta - 1u) / ncta);
     wide = wide || T.B > ncta;
     laneOff.push_back(laneH.size());
     laneH.resize(laneH.size() + T.B, kNoSlot);
-    for (const Active& a : A) {
+    for (Active& a : A) {
       PlanesEntry e{};
+      e.from = a.lane;
+      if (T.moved) a.lane = (uint32_t)(&a - A.data());
       e.slot = a.slot;
       e.t0 = a.tloc;
       e.clamp = a.req.clamp;

@@ -10,7 +10,11 @@ namespace axon {
 PlanesShape planes_serve_shape(uint32_t ncol, uint32_t B, int grid, uint32_t cols, uint32_t want, PlanesCfg* c) {
   PlanesShape s{};
   s.grid = grid;
-  s.direct = B <= kPlanesDirectB ? 1u : 0u;
+  // several teams' staged tiles don't stay in the L2 between steps (four networks of 4,096
+  // columns are 680 MB), so that reading what is needed pays up to larger batches (us per step of
+  // four teams, read / staged: 265 / 310 at 160 trajectories in the largest, 306 / 329 at 190, 380 / 345 at 223)
+  const bool teams = cols > (ncol + (uint32_t)grid - 1u) / (uint32_t)grid;
+  s.direct = B <= (teams ? 192u : kPlanesDirectB) ? 1u : 0u;
   s.smem = planes_fit(ncol, B, s.direct != 0u, true, cols, want, c);
   return s;
 }

@@ -93,3 +93,32 @@ def test_clamped_steps(clamp, B):
     net, pats = trained(incols=72)
     same(net, cues_of(net, pats, B, clamp), 8, clamp)
     net.close()
+
+
+# a server whose trajectories end at different steps moves the others to lower lanes: whole blocks of
+# staged and of directly read launches, small batches, and columns recomputed in the step of the move
+@pytest.mark.parametrize("kw,unit", [(dict(), 1), (dict(target=250), 1), (dict(incols=20, k=0), 1), (dict(), 12)])
+def test_server_moves_lanes(kw, unit):
+    net, pats = trained(**kw)
+    other, _ = trained(seed=1, **kw)
+    rng = np.random.default_rng(3)
+    reqs = []
+    for tag in range(450):
+        cols = np.sort(rng.choice(pats[tag % len(pats)], int(rng.integers(1, len(pats[0]) + 1)), replace=False)).astype(np.uint32)
+        reqs.append((int(tag % 9 == 0), cols, unit * int(rng.integers(1, 1 + 36 // unit))))
+    with ax.Server([net, other], 64 << 20) as srv:
+        at = ax.clock_s() + 0.02  # all together
+        for tag, (i, cols, free) in enumerate(reqs):
+            srv.submit(i, cols, 4, free, tag, at)
+        srv.wait_idle(120)
+        got = {res["tag"]: spikes for res, spikes in srv.poll(len(reqs))}
+    for free in sorted({f for _, _, f in reqs}):
+        for i, n in enumerate((net, other)):
+            tags = [t for t, (j, _, f) in enumerate(reqs) if j == i and f == free]
+            if tags:
+                cues = np.stack([ax.clamp_words(reqs[t][1], n.ncol) for t in tags])
+                want = n.recall(cues, 4 + free, 4, method="plain")["final"]
+                for t, w in zip(tags, want):
+                    assert np.array_equal(got[t], w), t
+    net.close()
+    other.close()
