@@ -75,6 +75,7 @@ struct PlanesDev {
   const PlanesTeam* teams;  // by cta0, covering the grid
   const PlanesEntry* entries;
   const uint32_t* cues;
+  uint32_t* teamNs;         // [nteams] duration of the launch on each team's first CTA
   uint32_t nteams;
 };
 

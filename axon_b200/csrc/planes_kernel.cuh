@@ -559,6 +559,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
                                                                      const __grid_constant__ PlanesCfg c) {
   extern __shared__ __align__(128) uint32_t sm[];
   uint32_t team = 0;
+  const uint64_t began = SERVE && threadIdx.x == 0 ? globaltimer_ns() : 0ull;
   if (SERVE)
     while (team + 1u < d.nteams && blockIdx.x >= d.teams[team + 1u].cta0) ++team;
   PlanesNet netS{};
@@ -1047,6 +1048,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
     if (!grid_barrier(net.bar, d.err, G, epoch++, c.waitNs, sMisc)) { drain(); return; }
   }
   drain();
+  if (SERVE && cta == 0u && tid == 0) d.teamNs[team] = (uint32_t)(globaltimer_ns() - began);
 }
 
 

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
+#include <cmath>
 #include <cstring>
 #include <deque>
 #include <mutex>
@@ -108,6 +109,8 @@ struct axon_server {
   PlanesDev pdev{};
   PlanesCfg pcfg{};
   uint32_t* actMem = nullptr;                   // activity words, [net][2][ngrp][kServeMaxB / 32]
+  std::vector<uint32_t> teamNet;                // the networks of a launch's teams
+  std::vector<double> netCost;                  // per network: cost of a trajectory, relative to the others'
   std::vector<uint32_t> netPar;                 // per network: parity that its next step reads
   std::vector<std::vector<uint32_t>> laneUsed;  // per network: bitmap of the lanes in use
   std::vector<PlanesEntry> pentH;
@@ -239,7 +242,7 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
 axon_status axon_server::start_planes(uint64_t memBytes) {
   const uint32_t n = (uint32_t)nets.size(), ngrp = ncol / 8u, ncw = ncol / 32u;
   const size_t actBytes = al(2ull * ngrp * (kServeMaxB / 32u) * 4);
-  const uint64_t fixed = n * actBytes + al(n * sizeof(PlanesTeam)) + al(n * 128) + al((size_t)n * kServeMaxB * 4) + 2048;
+  const uint64_t fixed = n * actBytes + al(n * sizeof(PlanesTeam)) + al(n * 128) + al((size_t)n * kServeMaxB * 4) + 3072;
   const size_t recB = (size_t)(ngrp + ncol) * 16, planeB = (size_t)ncol * 64, candB = (size_t)ncw * 4, drvB = (size_t)ncol * 4;
   const size_t perSlot = recB + planeB + candB + drvB + 8 + (size_t)ncol * 4 + sizeof(PlanesEntry) + (size_t)incols * 4;
   if (memBytes <= fixed + perSlot + 64) return set_error(AXON_EINVAL, "memory budget below one trajectory slot");
@@ -250,7 +253,7 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
                al((size_t)n * kServeMaxB * 4) + al((size_t)nslots * incols * 4);
   size_t off = 0;
   auto place = [&](size_t bytes) { const size_t o = off; off += al(bytes); return o; };
-  const size_t oErr = place(64), oAct = place(n * actBytes), oCand = place(nslots * candB), oTh = place(nslots * 8ull),
+  const size_t oErr = place(64 + n * 4ull), oAct = place(n * actBytes), oCand = place(nslots * candB), oTh = place(nslots * 8ull),
                oRec = place(nslots * recB), oPlane = place(nslots * planeB), oDrv = place(nslots * drvB),
                oStage = place(stageBytes), oDone = place((size_t)nslots * ncol * 4);
   if (cudaMalloc(&dmem, off) != cudaSuccess) {
@@ -260,7 +263,7 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
   }
   CKS(cudaMallocHost(&hmem, stageBytes));
   CKS(cudaMallocHost(&hdone, (size_t)nslots * ncol * 4));
-  CKS(cudaMallocHost((void**)&herr, 64));
+  CKS(cudaMallocHost((void**)&herr, 64 + n * 4));
   CKS(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   for (auto& evp : ev)
     for (auto& e : evp) CKS(cudaEventCreate(&e));
@@ -287,6 +290,8 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
   for (uint32_t s = nslots; s-- > 0;) freeSlots.push_back(s);
   act.assign(n, {});
   netPar.assign(n, 0u);
+  netCost.assign(n, 1.0);
+  pdev.teamNs = (uint32_t*)(b + oErr) + 16;
   laneUsed.assign(n, std::vector<uint32_t>(kServeMaxB / 32u, 0u));
   th = std::thread([this] { loop(); });
   return AXON_OK;
@@ -384,17 +389,24 @@ axon_status axon_server::tick_planes() {
   pentH.clear();
   laneH.clear();
   cueH.clear();
-  // CTAs in proportion to a network's trajectories (plus a share for its tiles), one at least
-  uint32_t ndone = 0, cta = 0, left = nact, weightLeft = total + 16u * nact;
+  // CTAs in proportion to a network's trajectories (plus a share for its tiles) and to what they
+  // cost, one at least. A trajectory of a heavily loaded network costs up to twice that of a
+  // light one, and a launch lasts as long as its slowest team.
+  auto weigh = [&](uint32_t n) { return ((double)act[n].size() + 16.0) * netCost[n]; };
+  uint32_t ndone = 0, cta = 0, left = nact;
+  double weightLeft = 0.0;
+  for (uint32_t n = 0; n < (uint32_t)act.size(); ++n)
+    if (!act[n].empty()) weightLeft += weigh(n);
   const uint32_t grid = (uint32_t)sms;
   std::vector<size_t> laneOff;
   bool wide = false;  // a team has more trajectories than CTAs
   for (uint32_t n = 0; n < (uint32_t)act.size(); ++n) {
     std::vector<Active>& A = act[n];
     if (A.empty()) continue;
-    const uint32_t weight = (uint32_t)A.size() + 16u, room = grid - cta - (left - 1u);
+    const double weight = weigh(n);
+    const uint32_t room = grid - cta - (left - 1u);
     const uint32_t ncta = left == 1u ? grid - cta
-                                     : std::max(1u, std::min(room, (uint32_t)((uint64_t)(grid - cta) * weight / weightLeft)));
+                                     : std::max(1u, std::min(room, (uint32_t)((grid - cta) * weight / weightLeft + 0.5)));
     PlanesTeam T{};
     T.net.W3P = nets[n]->w3p;
     T.net.conn = nets[n]->d.conn;
@@ -478,11 +490,13 @@ axon_status axon_server::tick_planes() {
     if (st != AXON_OK) return st;
   }
   if (ndone) CKS(cudaMemcpyAsync(hdone, dev.doneBuf, (size_t)ndone * ncol * 4, cudaMemcpyDeviceToHost, stream));
-  CKS(cudaMemcpyAsync(herr, dev.err, 4, cudaMemcpyDeviceToHost, stream));
+  CKS(cudaMemcpyAsync(herr, dev.err, 64 + nt * 4, cudaMemcpyDeviceToHost, stream));
   pending.clear();
   uint32_t ei = 0;
+  teamNet.clear();
   for (uint32_t n = 0; n < (uint32_t)act.size(); ++n) {
     std::vector<Active>& A = act[n];
+    if (!A.empty()) teamNet.push_back(n);
     size_t w = 0;
     for (size_t i = 0; i < A.size(); ++i) {
       Active& a = A[i];
@@ -514,6 +528,14 @@ axon_status axon_server::tick_planes() {
   CKS(cudaStreamSynchronize(stream));
   stepS = (now_s() - t0) / steps;
   if (herr[0] != 0u) return set_error(AXON_ETIMEOUT, "a wait timed out in the serving kernel");
+  if (nt > 1u) {  // the teams' durations move their networks' costs halfway to equal durations
+    double mean = 0.0;
+    for (uint32_t i = 0; i < nt; ++i) mean += (double)herr[16 + i] * teamH[i].ncta / (double)cta;
+    for (uint32_t i = 0; mean > 0.0 && i < nt; ++i) {
+      double& f = netCost[teamNet[i]];
+      f = std::min(4.0, std::max(0.25, f * std::sqrt(std::max(herr[16 + i] / mean, 0.25))));
+    }
+  }
   return AXON_OK;
 }
 
