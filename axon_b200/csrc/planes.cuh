@@ -25,6 +25,11 @@ constexpr uint32_t kPlanesList = 384;               // gated columns it lists th
 constexpr int planes_threads(bool direct) { return direct ? 896 : 640; }
 
 constexpr uint32_t kPlanesDirectB = 160;            // most trajectories whose tiles are read through L2
+// up to this width every column with a drive is a candidate: storing their planes costs less than
+// recomputing gated columns after a threshold below the floor, which small networks meet often
+// (us of a 30-step call of 40 trajectories, bias off and on, floor / all: 256 columns 800 / 726 and
+// 1639 / 1076; 512: 806 / 671 and 922 / 869; 1,024: 740 / 772 and 1030 / 1042)
+constexpr uint32_t kPlanesAllCols = 512;
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 
 // A network and the team's words for it.

@@ -1076,6 +1076,9 @@ size_t planes_fit(uint32_t ncol, uint32_t B, bool direct, bool serve, uint32_t c
   // 4,096-column network: 21.3 / 24.5 / 27.3 / 30.5 with one lane, 18.1 / 21.0 / 24.6 / 31.5
   // with two, 16.6 / 19.6 / 26.6 / 32.7 with four)
   c->ls = B > 20u ? 0u : B > 10u ? 1u : 2u;
+  // more, too, where one would leave most of a CTA's warps without a task (two columns of a
+  // 256-column network and 40 trajectories are four tasks)
+  while (direct && c->ls < 2u && cols * ((B + 31u) / 32u << (c->ls + 1u)) <= 28u) ++c->ls;
   c->ns = c->nl = 0;
   c->nsl = 2;
   c->nll = 3;

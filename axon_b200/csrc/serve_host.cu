@@ -41,7 +41,7 @@ struct Request {
 struct Active {
   uint32_t slot;
   uint32_t tloc;
-  uint32_t lane;  // bit-plane form: the trajectory's lane of its network, kept for its life
+  uint32_t lane;  // bit-plane form: the trajectory's lane of its network
   Request req;
 };
 
@@ -285,6 +285,7 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
   dev.err = pdev.err;
   pcfg.ncol = ncol; pcfg.incols = incols; pcfg.k = cfg.k; pcfg.dthr = cfg.dthr; pcfg.mode = cfg.mode;
   pcfg.targetCols = cfg.targetCols; pcfg.topkPar = cfg.topkPar; pcfg.bst = cfg.bst; pcfg.waitNs = nets[0]->wait_ns;
+  pcfg.slabFull = ncol <= kPlanesAllCols ? 1u : 0u;
   CKS(planes_serve_prepare(pcfg));
   CKS(cudaStreamSynchronize(stream));
   for (uint32_t s = nslots; s-- > 0;) freeSlots.push_back(s);
@@ -379,19 +380,19 @@ axon_status axon_server::tick_planes() {
       if (gap > 0 && stepS > 0) steps = (uint32_t)std::min<double>(steps, 1.0 + gap / stepS);
     }
   }
-  uint32_t nact = 0, total = 0, maxB = 0, maxCols = 0;
+  uint32_t nact = 0, maxB = 0, maxCols = 0;
   for (const std::vector<Active>& A : act) {
     for (const Active& a : A) steps = std::min(steps, a.req.steps - a.tloc);
     nact += !A.empty();
-    total += (uint32_t)A.size();
   }
   teamH.clear();
   pentH.clear();
   laneH.clear();
   cueH.clear();
   // CTAs in proportion to a network's trajectories (plus a share for its tiles) and to what they
-  // cost, one at least. A trajectory of a heavily loaded network costs up to twice that of a
-  // light one, and a launch lasts as long as its slowest team.
+  // cost, one at least. A trajectory of a heavily loaded network costs more than that of a light
+  // one, and a launch lasts as long as its slowest team (3,000 requests to eight networks of
+  // loads 12 to 200, by number alone / with the measured costs: 72.4 / 67.8 ms).
   auto weigh = [&](uint32_t n) { return ((double)act[n].size() + 16.0) * netCost[n]; };
   uint32_t ndone = 0, cta = 0, left = nact;
   double weightLeft = 0.0;

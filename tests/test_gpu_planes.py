@@ -122,3 +122,14 @@ def test_server_moves_lanes(kw, unit):
                     assert np.array_equal(got[t], w), t
     net.close()
     other.close()
+
+
+# both sides of the width up to which every column with a drive is a candidate, and sorted tasks with
+# several lanes per trajectory (two columns per CTA)
+@pytest.mark.parametrize("ncol,target", [(256, 8), (512, 24), (544, 24), (544, 460)])
+@pytest.mark.parametrize("B", [40, 96])
+def test_small_networks(ncol, target, B):
+    net, pats = trained(ncol=ncol, incols=64, target=target, k=24, nstim=12, epochs=2)
+    same(net, cues_of(net, pats, B, B), 12, 3, use_bias=1)
+    same(net, cues_of(net, pats, B, B + 1), 12, 3, slab="floor_always")
+    net.close()
