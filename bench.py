@@ -698,14 +698,14 @@ def main() -> None:
                    "parallelism": f"replicas x{world}"},
         "oracle_match": match,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                     "traffic": measured_traffic("k_recall"), "peak_kind": pk,
+                     "traffic": measured_traffic("k_recall_planes"), "peak_kind": pk,
                      "note": "algorithmic bytes = 45 x (W3 128 MiB + every trajectory's spike vector in and out); "
-                             "the kernel is bound by the popcount (XU) pipe and issue, see profiles/"},
+                             "the kernel is bound by shared-memory wavefronts and logic operations, see profiles/"},
         "int_roofline": {"bound": "xu (popcount pipe)", "achieved": pops / (ms / 1e3), "unit": "popcounts/s",
                          "peak": peak_pops, "frac": pops / (ms / 1e3) / peak_pops,
                          "note": "the contraction's unavoidable 32-bit AND-popcounts (32 rows x nonzero spike words "
                                  "of every active (column, branch, trajectory)) per second, against 16 popcounts per SM "
-                                 "per clock at the sampled SM clock; ncu's XU-pipe utilisation is the same measure"},
+                                 "per clock at the sampled SM clock; the bit-plane kernel forms them without that pipe"},
         "cpu_baseline": cpu,
         "e2e": {"value": world * events / e2e_s, "unit": "synaptic events/s",
                 "h2d_bytes_per_step": int(B * INCOLS * 4),  # the cues' input columns: all the clamp reads
