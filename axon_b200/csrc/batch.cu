@@ -381,7 +381,11 @@ __global__ void __launch_bounds__(896, 1) k_recall(RecallDev d, RecallCfg c) {
     // next step's list lengths start at zero (last read in phase 1 of step t-1)
     if (blockIdx.x == 0)
       for (uint32_t g = tid; g < 2 * ngrp; g += blockDim.x) c1Out[g] = 0u;
-    for (uint32_t b = tid; b < B; b += blockDim.x) sFloor[b] = hist_floor(d.thPrev + b);  // read after the sync below
+    // thresholds by step parity: this step reads the last one's and writes its own, so that every
+    // part of a split trajectory sees the same value for the whole step
+    const uint32_t* thIn = d.thPrev + (size_t)(par ^ 1u) * B;
+    uint32_t* thOut = d.thPrev + (size_t)par * B;
+    for (uint32_t b = tid; b < B; b += blockDim.x) sFloor[b] = hist_floor(thIn + b);  // read after the sync below
 
     // ---------------- phase 1
     // thread 0 claims one item ahead: the claim's round trip overlaps the current item. After
@@ -721,7 +725,7 @@ __global__ void __launch_bounds__(896, 1) k_recall(RecallDev d, RecallCfg c) {
       const uint32_t theta = sCtl[8] >= c.targetCols
                                  ? recall_theta(sD, sH, sList, sCtl, incols, ncol, c.targetCols, c.topkPar, grp)
                                  : block_theta(sD, incols, ncol, c.targetCols, c.topkPar, sHist, sRed,
-                                               __ldcg(d.thPrev + b), grp);
+                                               __ldcg(thIn + b), grp);
       // this trajectory's histogram of step t+1 mod 3, last read two steps ago, is cleared
       // for phase 1 of the next step
       if (pi == 0u) {
@@ -825,7 +829,7 @@ __global__ void __launch_bounds__(896, 1) k_recall(RecallDev d, RecallCfg c) {
         }
       }
       if (grp.t == 0 && pi == 0u) {
-        __stcg(d.thPrev + b, theta);
+        __stcg(thOut + b, theta);
         if (d.theta && t + 1u == c.T) d.theta[b] = theta;
       }
       grp.sync();

@@ -1,0 +1,47 @@
+"""The batched readout outside the bit planes (facilitation, boosts of 256 and more, the tensor
+contraction): every trajectory equals the plain path."""
+import numpy as np
+import pytest
+
+import axon_b200 as ax
+
+pytestmark = pytest.mark.gpu
+
+
+def trained(seed=0, nstim=6, epochs=3, **kw):
+    base = dict(ax.CONFIG_C, ncol=256, incols=64, target=16, k=12)
+    base.update(kw)
+    net = ax.Network(base)
+    net.init(seed)
+    pats = ax.stimuli(seed, nstim, base["incols"], max(4, base["incols"] // 4))
+    for _ in range(epochs):
+        for p in range(nstim):
+            net.present(ax.load_stim(pats[p], 1.0, 1000 + p, net.ncol), 10, 5, True)
+    return net, pats
+
+
+def cues_of(net, pats, B):
+    keep = (1.0, 0.75, 0.5, 0.35, 0.25, 0.1, 0.0)
+    return np.stack([ax.load_stim(pats[b % len(pats)], keep[b % len(keep)], 4400 + b, net.ncol) for b in range(B)])
+
+
+def same(net, cues, T, clamp, **kw):
+    a = net.recall(cues, T, clamp, hist=True, stats=True, **kw)
+    plain = {k: v for k, v in kw.items() if k in ("use_bias", "ref_ball")}
+    b = net.recall(cues, T, clamp, hist=True, stats=True, method="plain", **plain)
+    a["stats"][:, 2] = b["stats"][:, 2] = 0  # branch coincidence: plain method only
+    for k in ("final", "hist", "stats"):
+        assert np.array_equal(a[k], b[k]), k
+    if a["drive_log"] is not None:
+        assert np.array_equal(a["drive_log"], b["drive_log"])
+
+
+# trajectories split over several groups of warps (one CTA per SM, 148 on a B200: batches just above a multiple
+# of it, and 512), whose thresholds fall below the recorded drives after the clamp
+@pytest.mark.parametrize("B", [3, 149, 300, 512])
+def test_split_trajectories(B):
+    net, pats = trained()
+    cues = cues_of(net, pats, B)
+    for slab in ("floor", "floor_always") * 3:
+        same(net, cues, 16, 4, contraction="tensor", slab=slab)
+    net.close()

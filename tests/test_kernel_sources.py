@@ -1,0 +1,25 @@
+"""Orderings in the kernels that no run can show to be missing: memory that one part of a
+launch writes while another still reads it, read from the sources."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "axon_b200" / "csrc"
+
+
+def code(name: str) -> str:
+    """A source file without its comments."""
+    src = re.sub(r"/\*.*?\*/", "", (CSRC / name).read_text(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", src)
+
+
+def test_recall_reads_no_threshold_that_the_step_writes():
+    """Several groups of warps select the threshold of a split trajectory, starting from its
+    previous one, while the group with its first part stores the new one: the select's passes
+    (and their barriers) depend on that value, so what a step reads is never what it writes."""
+    src = code("batch.cu")
+    select = src[src.index("const uint32_t reFloor"):]
+    read = {m for m in re.findall(r"__ldcg\(([\w.]+) \+ b\), grp\)", select)} | set(re.findall(r"hist_floor\(([\w.]+) \+ b\)", src))
+    written = set(re.findall(r"__stcg\(([\w.]+) \+ b, theta\)", select))
+    assert len(read) == len(written) == 1 and read.isdisjoint(written)
+    define = {v: re.search(rf"uint32_t\* {v} = d\.thPrev \+ \(size_t\)(\(par \^ 1u\)|par) \* B;", src).group(1) for v in read | written}
+    assert define[read.pop()] == "(par ^ 1u)" and define[written.pop()] == "par"
