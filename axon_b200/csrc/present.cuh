@@ -208,7 +208,8 @@ struct PresentCta {
           __syncwarp();
           if (on) {
             const uint32_t r = (uint32_t)__popc(active & ((1u << lane) - 1u));
-            fence_proxy_async_smem();
+            if (LEARN) fence_proxy_async_all();
+            else fence_proxy_async_smem();
             bulk_g2s(sPool + (size_t)(slot0 + r) * kTileU4, d.W3 + ((size_t)cc * kNslot + lane) * kTileU4, 1024u, mb);
           }
         }
@@ -383,6 +384,7 @@ struct PresentCta {
             __stcg(d.W2 + base + 32 * j, p2[j]);
             __stcg(d.W3 + base + 32 * j, p3[j]);
           }
+          fence_proxy_async_all();  // the next step copies W3 tiles in bulk (async proxy)
           if (nLTP) atomicAdd(sLTP + slot * 32u + lane, nLTP);
           if (nLTD) atomicAdd(sLTD + slot * 32u + lane, nLTD);
         }

@@ -23,3 +23,19 @@ def test_recall_reads_no_threshold_that_the_step_writes():
     assert len(read) == len(written) == 1 and read.isdisjoint(written)
     define = {v: re.search(rf"uint32_t\* {v} = d\.thPrev \+ \(size_t\)(\(par \^ 1u\)|par) \* B;", src).group(1) for v in read | written}
     assert define[read.pop()] == "(par ^ 1u)" and define[written.pop()] == "par"
+
+
+def test_learned_tiles_are_fenced_before_they_are_copied():
+    """A learning step stores W3 tiles with ordinary stores that the next step reads by bulk
+    copies: between them, on the storing threads before the block barrier and on the copying
+    lanes before the copy, a proxy fence that covers global memory."""
+    src = code("present.cuh")
+    assert "fence.proxy.async;" in code("batch_common.cuh").split("fence_proxy_async_all()")[1].split("}")[0]
+    store = src.index("__stcg(d.W3")
+    assert "fence_proxy_async_all();" in src[store:src.index("__syncthreads()", store)]
+    copy = src.index("bulk_g2s(")
+    assert "if (LEARN) fence_proxy_async_all();" in src[src.rindex("if (on)", 0, copy):copy]
+    # no other kernel copies in bulk what the launch has stored
+    for name in sorted(p.name for p in CSRC.glob("*.cu*")):
+        if "bulk_g2s(" in code(name):
+            assert name == "present.cuh" or not re.search(r"__stcg\([^;]*\bW3", code(name)), name
