@@ -193,6 +193,10 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
     return set_error(AXON_EINVAL, "bad use_bias, method, contraction or slab");
   CK(cudaSetDevice(device));
 
+  // the batched forms use the reference assemblies for the member-drive log alone (the plain
+  // path logs into the network's own buffer when the caller passes none)
+  if (!driveLog && a.method != AXON_RECALL_PLAIN) refBall = nullptr;
+
   // ---- device views of the caller's arrays (copied in when they are host arrays)
   const size_t bn = (size_t)B * ncol;
   const uint32_t* dCues = cues;

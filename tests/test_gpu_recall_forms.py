@@ -1,9 +1,12 @@
 """The batched readout outside the bit planes (facilitation, boosts of 256 and more, the tensor
 contraction): every trajectory equals the plain path."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import axon_b200 as ax
+import axon_b200._capi as A
 
 pytestmark = pytest.mark.gpu
 
@@ -44,4 +47,19 @@ def test_split_trajectories(B):
     cues = cues_of(net, pats, B)
     for slab in ("floor", "floor_always") * 3:
         same(net, cues, 16, 4, contraction="tensor", slab=slab)
+    net.close()
+
+
+# every output of axon_recall is optional: reference assemblies without a log to write are accepted, and ignored
+@pytest.mark.parametrize("kw", [dict(), dict(boost=300), dict(facil=7), dict(boost=2000)])
+@pytest.mark.parametrize("contraction", [0, 1])
+def test_assemblies_without_a_log(kw, contraction):
+    net, pats = trained(**kw)
+    cues = cues_of(net, pats, 5)
+    want = net.recall(cues, 12, 4, method="plain")["final"]
+    got, ref = np.zeros_like(cues), np.full_like(cues, 0xFFFFFFFF)
+    for method in (0, 1):
+        a = A.RecallArgs(T=12, clamp_steps=4, method=method, contraction=contraction)
+        A.check(A.lib().axon_recall(net._h, A.u32(cues), 5, C.byref(a), A.u32(ref), A.u32(got), None, None, None, None))
+        assert np.array_equal(got, want)
     net.close()
