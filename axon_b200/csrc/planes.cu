@@ -2,6 +2,7 @@
 // readout itself is in planes_kernel.cuh.
 #include <cstdint>
 
+#include "plain.cuh"
 #include "planes_kernel.cuh"
 
 namespace axon {
@@ -62,7 +63,9 @@ PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c) {
 
 cudaError_t planes_max_blocks_per_sm(const PlanesCfg& c, const PlanesShape& s, int* out) {
   const void* fn = planes_fn<false>(c, s.direct);
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  // the limit is the process's, not the launch's: always the most a CTA can have, so that another
+  // thread's smaller call cannot lower it between this one and its launch
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, planes_threads(s.direct != 0u), s.smem);
 }

@@ -16,6 +16,7 @@
 #include <cstdint>
 
 #include "axon_device.cuh"
+#include "plain.cuh"
 #include "serve.cuh"
 #include "theta.cuh"
 
@@ -231,8 +232,10 @@ size_t serve_emit_smem_bytes(uint32_t ncol, uint32_t incols) {
   return (3ull * ncol + ((incols + 3u) & ~3u) + 256 + 192 + kEmitChunk * 32ull + 4) * 4;
 }
 
-cudaError_t serve_prepare(size_t emitSmem) {
-  return cudaFuncSetAttribute(k_serve_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emitSmem);
+// The limit is the process's: the most a CTA can have, so that a server of narrower networks
+// does not lower it under one that runs.
+cudaError_t serve_prepare() {
+  return cudaFuncSetAttribute(k_serve_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
 }
 
 // list lengths of the next tick start at zero (every network, parity par ^ 1)

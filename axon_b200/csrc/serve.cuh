@@ -92,7 +92,7 @@ size_t serve_emit_smem_bytes(uint32_t ncol, uint32_t incols);
 size_t serve_batched_smem_bytes(uint32_t packed);
 // most trajectories per network for which the batched drive keeps two counter buffers
 uint32_t serve_batched_dacc_maxb(uint32_t packed);
-cudaError_t serve_prepare(size_t emitSmem);
+cudaError_t serve_prepare();
 cudaError_t serve_batched_prepare(uint32_t packed);
 // drive kernels of one tick (gather for the groups, batched for the batched networks)
 cudaError_t launch_serve_drive(const ServeDev& d, const ServeCfg& c, int sms, bool gather, bool batched,

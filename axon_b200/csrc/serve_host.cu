@@ -227,7 +227,7 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
   dev.nactw = serve_nactw(ncol);
   dev.waitNs = n0->wait_ns;
   emitSmem = serve_emit_smem_bytes(ncol, incols);
-  CKS(serve_prepare(emitSmem));
+  CKS(serve_prepare());
   CKS(serve_batched_prepare(packed));
   CKS(cudaStreamSynchronize(stream));
   for (uint32_t s = nslots; s-- > 0;) freeSlots.push_back(s);

@@ -3,6 +3,7 @@
 // CTAs with a barrier of its own.
 #include <cstdint>
 
+#include "plain.cuh"
 #include "planes_kernel.cuh"
 
 namespace axon {
@@ -22,7 +23,7 @@ PlanesShape planes_serve_shape(uint32_t ncol, uint32_t B, int grid, uint32_t col
 cudaError_t planes_serve_prepare(const PlanesCfg& c) {
   for (uint32_t direct = 0; direct < 2u; ++direct) {
     const cudaError_t e = cudaFuncSetAttribute(planes_fn<true>(c, direct), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(227u * 1024u));
+                                               (int)kSmemLimitBytes);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
