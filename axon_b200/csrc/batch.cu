@@ -885,9 +885,7 @@ const void* recall_fn(uint32_t acc32, uint32_t lin, uint32_t mma) {
 cudaError_t recall_max_blocks_per_sm(int acc32, int threads, size_t smem, int* out) {
   for (uint32_t lin = 0; lin < 2; ++lin)
     for (uint32_t mma = 0; mma < 2; ++mma) {
-      // the process's limit: never lowered by one call under another thread's launch
-      cudaError_t e = cudaFuncSetAttribute(recall_fn(acc32, lin, mma), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kSmemLimitBytes);
+      const cudaError_t e = raise_smem_limit(recall_fn(acc32, lin, mma));
       if (e != cudaSuccess) return e;
     }
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, recall_fn(acc32, 1, 0), threads, smem);

@@ -504,8 +504,7 @@ static const void* multi_fn(int threads, int tiles, int cpw) {
 cudaError_t multi_max_blocks_per_sm(int threads, int tiles, int cpw, size_t smem, int* out) {
   const void* fn = multi_fn(threads, tiles, cpw);
   if (!fn) return cudaErrorInvalidValue;
-  // the process's limit: never lowered by one call under another thread's launch
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
+  const cudaError_t e = raise_smem_limit(fn);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, threads, smem);
 }

@@ -32,6 +32,15 @@ constexpr uint32_t kBarRegionWords = 64u + 3u * kHistWords;
 constexpr uint32_t kMaxColSlots = 64;      // column slots per CTA (32 warps x 2 columns)
 constexpr uint32_t kPresentMaxWarps = 28;  // k_present is compiled for 896 threads (72 registers)
 constexpr uint32_t kSmemLimitBytes = 227u * 1024u;
+// Sets a kernel's dynamic shared-memory limit to the most a CTA can have. The limit is the
+// process's, not the launch's: set to one call's size it would refuse a larger launch that
+// another thread or a running server has prepared.
+inline cudaError_t raise_smem_limit(const void* fn) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemLimitBytes - a.sharedSizeBytes));
+}
 struct PresentSmem {
   uint32_t poolWord;   // first word of the pool
   uint32_t poolTiles;  // 1 KiB W3 tiles the pool holds

@@ -63,9 +63,7 @@ PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c) {
 
 cudaError_t planes_max_blocks_per_sm(const PlanesCfg& c, const PlanesShape& s, int* out) {
   const void* fn = planes_fn<false>(c, s.direct);
-  // the limit is the process's, not the launch's: always the most a CTA can have, so that another
-  // thread's smaller call cannot lower it between this one and its launch
-  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
+  const cudaError_t e = raise_smem_limit(fn);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, fn, planes_threads(s.direct != 0u), s.smem);
 }

@@ -232,11 +232,7 @@ size_t serve_emit_smem_bytes(uint32_t ncol, uint32_t incols) {
   return (3ull * ncol + ((incols + 3u) & ~3u) + 256 + 192 + kEmitChunk * 32ull + 4) * 4;
 }
 
-// The limit is the process's: the most a CTA can have, so that a server of narrower networks
-// does not lower it under one that runs.
-cudaError_t serve_prepare() {
-  return cudaFuncSetAttribute(k_serve_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimitBytes);
-}
+cudaError_t serve_prepare() { return raise_smem_limit((const void*)k_serve_emit); }
 
 // list lengths of the next tick start at zero (every network, parity par ^ 1)
 __global__ void k_serve_zero_counts(ServeDev d, uint32_t nnets, uint32_t ngrp) {

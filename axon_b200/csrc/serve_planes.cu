@@ -22,8 +22,7 @@ PlanesShape planes_serve_shape(uint32_t ncol, uint32_t B, int grid, uint32_t col
 
 cudaError_t planes_serve_prepare(const PlanesCfg& c) {
   for (uint32_t direct = 0; direct < 2u; ++direct) {
-    const cudaError_t e = cudaFuncSetAttribute(planes_fn<true>(c, direct), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)kSmemLimitBytes);
+    const cudaError_t e = raise_smem_limit(planes_fn<true>(c, direct));
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
