@@ -89,6 +89,8 @@ struct axon_net {
   uint32_t* w3p = nullptr;      // W3 in the bit-plane layout (planes.cuh), rebuilt when weights change
   bool w3p_valid = false;
   axon_status ensure_w3p();
+  bool w3p_served = false;      // a server has read it: not given back before the network ends
+  void drop_w3p();              // gives its memory back, for a form that needs less
   axon_status recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
                             uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog);
   // the batched readout as a captured CUDA graph, with the arguments it was captured for

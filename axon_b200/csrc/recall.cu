@@ -61,6 +61,13 @@ axon_status axon_net::ensure_w3p() {
   return AXON_OK;
 }
 
+void axon_net::drop_w3p() {
+  if (!w3p || w3p_served) return;
+  cudaFree(w3p);
+  w3p = nullptr;
+  w3p_valid = false;
+}
+
 namespace {
 size_t al(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 }  // namespace
@@ -72,6 +79,8 @@ bool axon::planes_config(const axon_cfg& cfg) {
 
 axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
                                     uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog) {
+  axon_status st = ensure_w3p();
+  if (st != AXON_OK) return st;
   const uint32_t ngrp = ncol / 8u, nl = (B + kPlanesMaxB - 1u) / kPlanesMaxB, Bc = (B + nl - 1u) / nl;  // launches, trajectories of one
   const PresentCfg pc = present_cfg(a.T, a.clamp_steps, false, a.use_bias);
   PlanesCfg c{};
@@ -93,7 +102,7 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   planes_shape(ncol, Bc, sm_count, &c);
   const size_t affBytes = c.aff && a.clamp_steps >= 2u && a.T >= 3u && cfg.incols % 8u == 0u ? al((size_t)ncol * nblk * 32 * 64) : 0;
   bool useAff = affBytes != 0;
-  axon_status st = scratch.ensure(need + affBytes);
+  st = scratch.ensure(need + affBytes);
   if (st != AXON_OK && useAff) {
     useAff = false;
     st = scratch.ensure(need);
@@ -230,6 +239,13 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
   if (dStats) CK(cudaMemsetAsync(dStats, 0, (size_t)B * 4096, stream));
 
   float gpu_ms = 0.f;
+  bool planes = a.method == AXON_RECALL_BATCHED && a.contraction == AXON_CONTRACT_POPC && planes_config(cfg);
+  if (planes) {
+    const axon_status st = recall_planes(dCues, B, a, dRef, dFinal, dHist, dStats, dLog);
+    if (st != AXON_OK && st != AXON_ENOMEM) return st;
+    planes = st == AXON_OK;
+    if (!planes) drop_w3p();  // its layout or scratch does not fit the device's memory: the older form needs less
+  }
   if (a.method == AXON_RECALL_PLAIN) {
     // one persistent presentation launch per trajectory
     const size_t zbytes = al(ncol * 4);
@@ -252,10 +268,7 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
       CK(launch_present(dd, pc, shape, stream));
     }
     CK(cudaEventRecord(ev1, stream));
-  } else if (a.contraction == AXON_CONTRACT_POPC && planes_config(cfg) && ensure_w3p() == AXON_OK) {
-    const axon_status st = recall_planes(dCues, B, a, dRef, dFinal, dHist, dStats, dLog);
-    if (st != AXON_OK) return st;
-  } else {
+  } else if (!planes) {
     if (ncol > 8192) return set_error(AXON_EINVAL, "batched recall supports ncol <= 8192; use the plain method");
     axon_status st = ensure_w3b();
     if (st != AXON_OK) return st;

@@ -170,7 +170,12 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
     planes = nets[i]->ensure_w3p() == AXON_OK;
     if (planes) CKS(cudaStreamSynchronize(nets[i]->stream));
   }
-  if (planes) return start_planes(memBytes);
+  if (planes) {
+    const axon_status st = start_planes(memBytes);
+    if (st != AXON_ENOMEM) return st;
+    planes = false;
+  }
+  for (axon_net* x : nets) x->drop_w3p();  // the layouts that did fit leave room for the older, smaller ones
   for (axon_net* x : nets) {  // the batched tile layout of every served network
     axon_status st = x->ensure_w3b();
     if (st != AXON_OK) return st;
@@ -294,6 +299,7 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
   netCost.assign(n, 1.0);
   pdev.teamNs = (uint32_t*)(b + oErr) + 16;
   laneUsed.assign(n, std::vector<uint32_t>(kServeMaxB / 32u, 0u));
+  for (axon_net* x : nets) x->w3p_served = true;
   th = std::thread([this] { loop(); });
   return AXON_OK;
 }
