@@ -28,7 +28,7 @@ __device__ __forceinline__ uint32_t popc4(uint4 a, uint4 b) {
 
 // ---------------------------------------------------------------- bit-serial counters
 // 4-bit counters held as 4 bitplanes; one 32-bit word per plane = 32 synapses.
-// Saturating +1 / -1 and the symmetric clip of src/axon.mm:371-420.
+// Saturating +1 / -1 of src/axon.mm:371-388 (the clip is in learn.cuh).
 __device__ __forceinline__ void bs_inc(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3, uint32_t m) {
   uint32_t c = m, t;
   t = a0 ^ c; c &= a0; a0 = t;
@@ -44,42 +44,6 @@ __device__ __forceinline__ void bs_dec(uint32_t& a0, uint32_t& a1, uint32_t& a2,
   t = a2 ^ b; b &= ~a2; a2 = t;
   t = a3 ^ b; b &= ~a3; a3 = t;
   a0 &= ~b; a1 &= ~b; a2 &= ~b; a3 &= ~b;
-}
-// synapses whose value is < K (lt) and > K (gt); K in 0..15
-__device__ __forceinline__ uint32_t bs_lt(uint32_t a3, uint32_t a2, uint32_t a1, uint32_t a0, uint32_t K) {
-  uint32_t lt = 0, eq = kFull;
-  if ((K >> 3) & 1u) lt |= eq & ~a3;
-  eq &= ((K >> 3) & 1u) ? a3 : ~a3;
-  if ((K >> 2) & 1u) lt |= eq & ~a2;
-  eq &= ((K >> 2) & 1u) ? a2 : ~a2;
-  if ((K >> 1) & 1u) lt |= eq & ~a1;
-  eq &= ((K >> 1) & 1u) ? a1 : ~a1;
-  if (K & 1u) lt |= eq & ~a0;
-  return lt;
-}
-__device__ __forceinline__ uint32_t bs_gt(uint32_t a3, uint32_t a2, uint32_t a1, uint32_t a0, uint32_t K) {
-  uint32_t gt = 0, eq = kFull;
-  if (!((K >> 3) & 1u)) gt |= eq & a3;
-  eq &= ((K >> 3) & 1u) ? a3 : ~a3;
-  if (!((K >> 2) & 1u)) gt |= eq & a2;
-  eq &= ((K >> 2) & 1u) ? a2 : ~a2;
-  if (!((K >> 1) & 1u)) gt |= eq & a1;
-  eq &= ((K >> 1) & 1u) ? a1 : ~a1;
-  if (!(K & 1u)) gt |= eq & a0;
-  return gt;
-}
-__device__ __forceinline__ void bs_set(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3, uint32_t m, uint32_t C) {
-  const uint32_t keep = ~m;
-  a0 = (a0 & keep) | ((C & 1u) ? m : 0u);
-  a1 = (a1 & keep) | ((C & 2u) ? m : 0u);
-  a2 = (a2 & keep) | ((C & 4u) ? m : 0u);
-  a3 = (a3 & keep) | ((C & 8u) ? m : 0u);
-}
-__device__ __forceinline__ void bs_clip(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3, uint32_t lo, uint32_t hi) {
-  const uint32_t l = bs_lt(a3, a2, a1, a0, lo);
-  const uint32_t g = bs_gt(a3, a2, a1, a0, hi);
-  bs_set(a0, a1, a2, a3, l, lo);
-  bs_set(a0, a1, a2, a3, g, hi);
 }
 
 // ---------------------------------------------------------------- exact k-of-32

@@ -145,6 +145,7 @@ axon_status axon_kwtatest(int device, const uint32_t* v, const uint32_t* k, uint
   cudaError_t e = cudaMemcpy(d, v, (size_t)n * 32u * 4u, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + (size_t)n * 32u, k, (size_t)n * 4u, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = launch_kwtatest(d, d + (size_t)n * 32u, d + (size_t)n * 33u, n, 0);
+  if (e == cudaSuccess) e = launch_kwtatest_planes(d, d + (size_t)n * 32u, d + (size_t)n * 33u, n, 0);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(out, d + (size_t)n * 33u, (size_t)n * 12u, cudaMemcpyDeviceToHost);
   cudaFree(d);

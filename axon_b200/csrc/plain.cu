@@ -25,6 +25,7 @@
 
 #include "axon_device.cuh"
 #include "batch_common.cuh"
+#include "learn.cuh"
 #include "plain.cuh"
 #include "present.cuh"
 
@@ -252,12 +253,12 @@ __global__ void k_bstest(uint32_t* A0, uint32_t* A1, uint32_t* A2, uint32_t* A3,
   uint32_t a0 = A0[g], a1 = A1[g], a2 = A2[g], a3 = A3[g];
   if (op == 0u) bs_inc(a0, a1, a2, a3, M[g]);
   else if (op == 1u) bs_dec(a0, a1, a2, a3, M[g]);
-  else bs_clip(a0, a1, a2, a3, lo, hi);
+  else band_clip(a0, a1, a2, a3, band_of(lo, hi));  // as learn_word does
   A0[g] = a0; A1[g] = a1; A2[g] = a2; A3[g] = a3;
 }
 
-// The kernels' k-of-32 (warp_kwta, src/axon.mm:134-144) on n columns of 32 values, one warp
-// per column: out[3i..3i+2] = winners ballot, vk, vk1.
+// The k-of-32 of the kernels with a lane per neuron (warp_kwta, src/axon.mm:134-144) on n columns
+// of 32 values, one warp per column: out[3i..3i+2] = winners ballot, vk, vk1.
 __global__ void k_kwtatest(const uint32_t* v, const uint32_t* k, uint32_t* out, uint32_t n) {
   const uint32_t lane = threadIdx.x & 31u, col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (col >= n) return;  // whole warps

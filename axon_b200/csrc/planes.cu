@@ -49,6 +49,23 @@ __global__ void k_planes_aux(const uint32_t* bias, uint32_t biasShift, const uin
   }
 }
 
+// The known-answer hook's second half, after k_kwtatest: where the values fit the drive planes,
+// plane_kwta has to give the same winners and values; a column where it does not gets its ballot
+// inverted. (With no winners, or all, the readout asks for no values.)
+__global__ void k_kwtatest_planes(const uint32_t* v, const uint32_t* k, uint32_t* out, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u, col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (col >= n) return;  // whole warps
+  const uint32_t x = v[(size_t)col * 32u + lane], kk = k[col];
+  if (__any_sync(kFull, x >> kPlanes)) return;
+  uint32_t D[kPlanes], vk, vk1;
+#pragma unroll
+  for (uint32_t i = 0; i < kPlanes; ++i) D[i] = __ballot_sync(kFull, (x >> i) & 1u);
+  const uint32_t ball = plane_kwta(D, kk, true, vk, vk1);
+  const bool same = ball == out[3u * col] && (kk == 0u || (vk == out[3u * col + 1u] && vk1 == out[3u * col + 2u]));
+  __syncwarp();
+  if (lane == 0 && !same) out[3u * col] = ~ball;
+}
+
 PlanesShape planes_shape(uint32_t ncol, uint32_t B, int sms, PlanesCfg* c) {
   PlanesShape s{};
   s.grid = sms;
@@ -71,6 +88,11 @@ cudaError_t planes_max_blocks_per_sm(const PlanesCfg& c, const PlanesShape& s, i
 cudaError_t launch_recall_planes(const PlanesDev& d, const PlanesCfg& c, const PlanesShape& s, cudaStream_t st) {
   void* args[] = {(void*)&d, (void*)&c};
   return cudaLaunchCooperativeKernel(planes_fn<false>(c, s.direct), dim3(s.grid), dim3(planes_threads(s.direct != 0u)), args, s.smem, st);
+}
+
+cudaError_t launch_kwtatest_planes(const uint32_t* v, const uint32_t* k, uint32_t* out, uint32_t n, cudaStream_t st) {
+  k_kwtatest_planes<<<(n + 7u) / 8u, 256, 0, st>>>(v, k, out, n);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_make_w3p(const uint4* W3, uint32_t* W3P, uint32_t ncol, cudaStream_t st) {

@@ -116,5 +116,7 @@ cudaError_t launch_make_w3p(const uint4* W3, uint32_t* W3P, uint32_t ncol, cudaS
 // bias planes and multiplicity masks (either output may be null)
 cudaError_t launch_planes_aux(const uint32_t* bias, uint32_t biasShift, const uint32_t* mult, uint32_t* biasP,
                               uint32_t* multM, uint32_t ncol, cudaStream_t st);
+// checks plane_kwta on columns that k_kwtatest has answered (see there)
+cudaError_t launch_kwtatest_planes(const uint32_t* v, const uint32_t* k, uint32_t* out, uint32_t n, cudaStream_t st);
 
 }  // namespace axon

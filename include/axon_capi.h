@@ -126,12 +126,15 @@ axon_status axon_untouched(axon_net* net, uint32_t* out_n);
 axon_status axon_wdiag(axon_net* net, const uint32_t* memb, const uint32_t* asm_spk,
                        uint32_t nstim, uint32_t sel, uint32_t hist48[48]);
 /* Bit-serial known-answer hook: k_bstest, src/axon.mm:424-434. a0..a3 and m hold n
- * words each (n a multiple of 4); op 0 inc, 1 dec, 2 clip [lo,hi]; planes updated. */
+ * words each (n a multiple of 4); op 0 inc, 1 dec, 2 clip [lo,hi]; planes updated by the functions
+ * that the learning kernels call. */
 axon_status axon_bstest(int device, uint32_t op, uint32_t lo, uint32_t hi, uint32_t* a0,
                         uint32_t* a1, uint32_t* a2, uint32_t* a3, const uint32_t* m, uint64_t n);
 /* k-of-32 known-answer hook: the kernels' exact k-WTA ranking (kwta_ballot_margin,
  * src/axon.mm:134-144) on n columns: v holds 32 values per column, k one k per column;
- * out receives per column the winners ballot, vk and vk1 (3 words). */
+ * out receives per column the winners ballot, vk and vk1 (3 words). Both of the kernels' forms run:
+ * a lane per neuron, and for values below 2^14 also the bit planes of the batched readout and the
+ * server; a column on which they differ gets an inverted ballot. */
 axon_status axon_kwtatest(int device, const uint32_t* v, const uint32_t* k, uint32_t* out, uint32_t n);
 
 /* Stimulus patterns: `nstim` rows of `stimcols` input-column indices, drawn as

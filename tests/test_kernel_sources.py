@@ -1,5 +1,6 @@
-"""Orderings in the kernels that no run can show to be missing: memory that one part of a
-launch writes while another still reads it, read from the sources."""
+"""What no run can show to be missing, read from the sources: the order of accesses to memory that
+one part of a launch writes and another reads, and that the known-answer hooks run the functions
+that the kernels run."""
 import re
 from pathlib import Path
 
@@ -39,3 +40,24 @@ def test_learned_tiles_are_fenced_before_they_are_copied():
     for name in sorted(p.name for p in CSRC.glob("*.cu*")):
         if "bulk_g2s(" in code(name):
             assert name == "present.cuh" or not re.search(r"__stcg\([^;]*\bW3", code(name)), name
+
+
+def calls(src: str, name: str, function: str) -> bool:
+    """Whether the body of the function `name` in src calls `function`."""
+    at = re.search(rf"\b{name}\([^;{{]*\)\s*{{", src).end()
+    depth, end = 1, at
+    while depth:
+        depth += {"{": 1, "}": -1}.get(src[end], 0)
+        end += 1
+    return re.search(rf"\b{function}[<(]", src[at:end]) is not None
+
+
+def test_known_answer_hooks_run_the_kernels_functions():
+    for f in ("bs_inc", "bs_dec", "band_clip"):
+        assert calls(code("learn.cuh"), "learn_word", f) and calls(code("plain.cu"), "k_bstest", f), f
+    assert calls(code("plain.cu"), "k_kwtatest", "warp_kwta")
+    assert calls(code("planes.cu"), "k_kwtatest_planes", "plane_kwta")
+    assert calls(code("planes_kernel.cuh"), "k_recall_planes", "plane_kwta")
+    capi = code("capi.cu")
+    for hook in ("launch_bstest", "launch_kwtatest", "launch_kwtatest_planes"):
+        assert f"{hook}(" in capi, hook
