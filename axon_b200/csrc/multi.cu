@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_multi_pool(MultiDe
   NetDev* sNet = reinterpret_cast<NetDev*>(sm + L.poolWord + (L.poolTiles - 1u) * 256u);
   PresentCfg* sCfg = reinterpret_cast<PresentCfg*>(sNet + 1);
   static_assert(sizeof(NetDev) + sizeof(PresentCfg) <= 1024u, "the two structures share one tile");
-  PresentCta<CPW> w;
-  w.init(sm, c.ncol, c.incols, tm);
+  PresentCta<CPW, true> w;
+  w.init(c.ncol, c.incols, tm);
   if (tid == 0) {
     PresentCfg p{};
     p.ncol = c.ncol; p.incols = c.incols; p.dthr = c.dthr; p.boost = c.boost; p.mode = c.mode;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_multi_pool(MultiDe
       sNet->err = m.err;
     }
     __syncthreads();
-    w.load(*sNet);
+    w.load(*sNet, tm);
     bool learned = false;
     for (uint32_t pi = 0; pi < nprog; ++pi) {
       if (tid == 0) {
@@ -460,16 +460,16 @@ __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_multi_pool(MultiDe
         sCfg->k = p.k; sCfg->facil = p.facil;
       }
       __syncthreads();
-      w.begin(*sNet);
+      w.begin(*sNet, tm);
       __syncthreads();
       const bool learn = sCfg->learn != 0u;
       if (!(learn ? w.template steps<true>(*sNet, *sCfg, tm, g) : w.template steps<false>(*sNet, *sCfg, tm, g))) return;
-      w.end(*sNet, sCfg->T);
+      w.end(*sNet, tm, sCfg->T);
       g += sCfg->T;
       learned = learned || learn;
       __syncthreads();
     }
-    if (learned) w.store_bias(*sNet);
+    if (learned) w.store_bias(*sNet, tm);
   }
   if (lane == 0 && w.nTiles) atomicAdd(m.work, (unsigned long long)w.nTiles);
   if (tid == 0 && w.nTasks) atomicAdd(m.work + 1, (unsigned long long)w.nTasks);

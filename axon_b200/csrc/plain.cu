@@ -33,17 +33,16 @@ namespace axon {
 
 template <int CPW, bool LEARN>
 __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, PresentCfg c) {
-  extern __shared__ __align__(16) uint32_t sm[];
   const PresentTeam tm{blockIdx.x, gridDim.x, c.ownWarps, present_smem_layout(c.ncol, c.incols, CPW).poolTiles, d.bar,
                        d.bar + 64};
-  PresentCta<CPW> w;
-  w.init(sm, c.ncol, c.incols, tm);
-  w.load(d);
-  w.begin(d);
+  PresentCta<CPW, false> w;
+  w.init(c.ncol, c.incols, tm);
+  w.begin(d, tm);
+  w.load(d, tm);
   __syncthreads();
   if (!w.template steps<LEARN>(d, c, tm, 0u)) return;
-  w.end(d, c.T);
-  if (LEARN) w.store_bias(d);
+  w.end(d, tm, c.T);
+  if (LEARN) w.store_bias(d, tm);
 }
 
 // ---------------------------------------------------------------- launch helpers

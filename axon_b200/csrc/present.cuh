@@ -21,53 +21,75 @@ struct PresentTeam {
   uint32_t *bar, *hist;  // barrier counter; three drive histograms
 };
 
-// A CTA's shared memory and the columns each of its warps owns, CPW per warp.
-template <int CPW>
+// A CTA's shared memory. Every function that uses it builds the map in place.
+struct PresentMap {
+  uint32_t *spk0, *spk1;   // spike vectors, ping-pong
+  uint32_t *act0, *act1;   // group-activity bits, ping-pong
+  uint32_t* stim;          // input clamp pattern
+  uint32_t* hist;          // the step's drive histogram (kHistWords)
+  uint32_t* flag;          // [0] barrier flag, [1] learning-task count, [2] candidates,
+                           // [3] tile-pool slots claimed, [4..7] threshold select
+  uint64_t* mbar;          // one per column slot (tile pool)
+  uint32_t* task;          // learning tasks: (column slot << 5) | branch
+  uint32_t* bbl;           // branch-NMDA masks of the learning columns
+  uint32_t *ltp, *ltd;     // per-neuron potentiation and depression counts of this step
+  uint32_t* firedL;        // spike ballot of each learning column
+  uint32_t* colL;          // its column index
+  uint32_t* mark;          // step+1 when the slot learns this step
+  uint32_t* bias;          // intrinsic bias of each owned neuron (slot * 32 + lane)
+  uint32_t* mul;           // assembly multiplicity of each owned neuron
+  uint32_t* ref;           // reference ball of each owned column
+  uint4* pool;             // phase A's tile pool; phase B reuses its start for
+  uint32_t *drv, *ball, *cand;  // the staged drives and ungated ballots of the current step, and the
+                                // drives of the threshold's histogram bin (up to ncol)
+};
+// maxCols: columns owned by the CTA
+__device__ __forceinline__ PresentMap present_map(uint32_t ncol, uint32_t incols, uint32_t maxCols, int cpw) {
+  extern __shared__ __align__(16) uint32_t sm[];
+  const uint32_t nactw = (((ncol / 8u + 31u) / 32u) + 3u) & ~3u;  // 16-byte multiple
+  PresentMap S;
+  S.spk0 = sm;
+  S.spk1 = sm + ncol;
+  S.act0 = sm + 2 * ncol;
+  S.act1 = S.act0 + nactw;
+  S.stim = S.act1 + nactw;
+  S.hist = S.stim + ((incols + 3u) & ~3u);
+  S.flag = S.hist + kHistWords;
+  S.mbar = reinterpret_cast<uint64_t*>(S.flag + 16);
+  S.task = S.flag + 16 + 2 * kMaxColSlots;
+  S.bbl = S.task + maxCols * 32;
+  S.ltp = S.bbl + maxCols * 32;
+  S.ltd = S.ltp + maxCols * 32;
+  S.firedL = S.ltd + maxCols * 32;
+  S.colL = S.firedL + maxCols;
+  S.mark = S.colL + maxCols;
+  S.bias = S.mark + maxCols;
+  S.mul = S.bias + maxCols * 32;
+  S.ref = S.mul + maxCols * 32;
+  S.drv = sm + present_smem_layout(ncol, incols, cpw).poolWord;
+  S.pool = reinterpret_cast<uint4*>(S.drv);
+  S.ball = S.drv + ncol;
+  S.cand = S.ball + ncol;
+  return S;
+}
+
+// The columns that each warp of a CTA owns, CPW per warp. MULTI: outputs may be absent and the
+// work is counted (the plain kernel always has them all).
+template <int CPW, bool MULTI>
 struct PresentCta {
-  uint32_t *sSpk0, *sSpk1, *sAct0, *sAct1, *sStim, *sHist, *sFlag, *sTask, *sBBL, *sLTP, *sLTD, *sFiredL, *sColL, *sMark,
-      *sBias, *sMul, *sRef, *sD, *sB, *sCand;
-  uint64_t* sMbar;
-  uint4* sPool;
-  uint32_t ncol, incols, nactw, maxCols;
+  uint32_t ncol, incols;
   uint32_t col[CPW], cn[CPW];
   uint32_t mph;  // bit i: phase parity of column slot i's mbarrier
   uint32_t nTiles, nTasks;  // W3 tiles this warp read, learning tasks of the CTA
 
   // once per launch
-  __device__ __forceinline__ void init(uint32_t* sm, uint32_t ncol_, uint32_t incols_, const PresentTeam& tm) {
+  __device__ __forceinline__ void init(uint32_t ncol_, uint32_t incols_, const PresentTeam& tm) {
     ncol = ncol_;
     incols = incols_;
-    const uint32_t ngrp = ncol / 8u, tid = threadIdx.x, warp = tid >> 5;
-    nactw = (((ngrp + 31u) / 32u) + 3u) & ~3u;  // 16-byte multiple
-    maxCols = tm.own * CPW;                     // columns owned by this CTA
-    const PresentSmem L = present_smem_layout(ncol, incols, CPW);
-    sSpk0 = sm;                    // spike vectors, ping-pong
-    sSpk1 = sm + ncol;
-    sAct0 = sm + 2 * ncol;         // group-activity bits, ping-pong
-    sAct1 = sAct0 + nactw;
-    sStim = sAct1 + nactw;         // input clamp pattern
-    sHist = sStim + ((incols + 3u) & ~3u);  // the step's drive histogram (kHistWords)
-    sFlag = sHist + kHistWords;    // [0] barrier flag, [1] learning-task count, [2] candidates,
-                                   // [3] tile-pool slots claimed, [4..7] threshold select
-    sMbar = reinterpret_cast<uint64_t*>(sFlag + 16);  // one per column slot (tile pool)
-    sTask = sFlag + 16 + 2 * kMaxColSlots;  // learning tasks: (column slot << 5) | branch
-    sBBL = sTask + maxCols * 32;   // branch-NMDA masks of the learning columns
-    sLTP = sBBL + maxCols * 32;    // per-neuron potentiation counts of this step
-    sLTD = sLTP + maxCols * 32;    // per-neuron depression counts
-    sFiredL = sLTD + maxCols * 32; // spike ballot of each learning column
-    sColL = sFiredL + maxCols;     // its column index
-    sMark = sColL + maxCols;       // step+1 when the slot learns this step
-    sBias = sMark + maxCols;       // intrinsic bias of each owned neuron (slot * 32 + lane)
-    sMul = sBias + maxCols * 32;   // assembly multiplicity of each owned neuron
-    sRef = sMul + maxCols * 32;    // reference ball of each owned column
-    // phase A's tile pool; phase B reuses its start for the staged drives, the ungated
-    // ballots and the threshold candidates
-    sPool = reinterpret_cast<uint4*>(sm + L.poolWord);
-    sD = sm + L.poolWord;          // staged drives of the current step
-    sB = sD + ncol;                // staged ungated ballots
-    sCand = sB + ncol;             // drives of the threshold's histogram bin (up to ncol)
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
-      for (uint32_t i = 0; i < maxCols; ++i) mbar_init(&sMbar[i], 1);
+      for (uint32_t i = 0; i < tm.own * CPW; ++i) mbar_init(&S.mbar[i], 1);
       fence_proxy_async_smem();
     }
     // columns are dealt to warps CTA-interleaved (column = warp * team + CTA): the clamped
@@ -81,7 +103,8 @@ struct PresentCta {
 
   // once per network: the owned columns' conn rows (lane = branch) in registers, the rest of
   // their per-neuron state in shared memory by column slot (warp * CPW + i)
-  __device__ __forceinline__ void load(const NetDev& d) {
+  __device__ __forceinline__ void load(const NetDev& d, const PresentTeam& tm) {
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < CPW; ++i) {
@@ -89,23 +112,25 @@ struct PresentCta {
       const uint32_t slot = warp * CPW + (uint32_t)i;
       if (col[i] < ncol) {
         cn[i] = d.conn[col[i] * kNslot + lane];
-        sBias[slot * 32u + lane] = d.bias[col[i] * 32u + lane];
-        sMul[slot * 32u + lane] = d.mult[col[i] * 32u + lane];
+        S.bias[slot * 32u + lane] = d.bias[col[i] * 32u + lane];
+        S.mul[slot * 32u + lane] = d.mult[col[i] * 32u + lane];
+        if (!MULTI && lane == 0) S.ref[slot] = d.refBall[col[i]];
       }
     }
   }
 
   // once per presentation, before a block barrier
-  __device__ __forceinline__ void begin(const NetDev& d) {
+  __device__ __forceinline__ void begin(const NetDev& d, const PresentTeam& tm) {
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    for (uint32_t i = tid; i < ncol; i += blockDim.x) sSpk0[i] = 0u;
-    for (uint32_t i = tid; i < nactw; i += blockDim.x) sAct0[i] = 0u;
-    for (uint32_t i = tid; i < maxCols; i += blockDim.x) sMark[i] = 0u;
-    if (tid == 0) sFlag[1] = sFlag[3] = 0u;
-    for (uint32_t i = tid; i < incols; i += blockDim.x) sStim[i] = d.stim[i];
+    for (uint32_t i = tid; i < ncol; i += blockDim.x) S.spk0[i] = 0u;
+    for (uint32_t i = tid; i < (uint32_t)(S.act1 - S.act0); i += blockDim.x) S.act0[i] = 0u;
+    for (uint32_t i = tid; i < tm.own * CPW; i += blockDim.x) S.mark[i] = 0u;
+    if (tid == 0) S.flag[1] = S.flag[3] = 0u;
+    for (uint32_t i = tid; i < incols; i += blockDim.x) S.stim[i] = d.stim[i];
 #pragma unroll
-    for (int i = 0; i < CPW; ++i)
-      if (col[i] < ncol && lane == 0) sRef[warp * CPW + (uint32_t)i] = d.refBall ? d.refBall[col[i]] : 0u;
+    for (int i = 0; MULTI && i < CPW; ++i)
+      if (col[i] < ncol && lane == 0) S.ref[warp * CPW + (uint32_t)i] = d.refBall ? d.refBall[col[i]] : 0u;
   }
 
   // The T steps; g0 = steps the team has run before (barrier epoch, exchange parity and
@@ -113,6 +138,11 @@ struct PresentCta {
   // carry none of the learning code's register pressure. Returns false when a grid wait gave up.
   template <bool LEARN>
   __device__ __forceinline__ bool steps(const NetDev& d, const PresentCfg& c, const PresentTeam& tm, uint32_t g0) {
+    // a readout takes the sizes from the kernel's parameters, and the shared-memory map from them, instead of
+    // holding them for the launch: a step of 2,080 columns takes 6.35 us (drive 2.21, spikes 1.82) against 6.47
+    // (2.25, 1.88). Learning is the other way round (a 10-step presentation of 4,096 columns 202 against 189 us)
+    const uint32_t ncol = MULTI || LEARN ? this->ncol : c.ncol, incols = MULTI || LEARN ? this->incols : c.incols;
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t ngrp = ncol / 8u, poolTiles = tm.poolTiles;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, wpb = blockDim.x >> 5;
     // branch term of k_drive (src/axon.mm:174-178): the count (modes 0, 1) plus, when the
@@ -140,20 +170,20 @@ struct PresentCta {
       }
       if (recur) {
         const uint32_t coinc = __reduce_add_sync(kFull, fired ? (uint32_t)__popc(bb[i]) : 0u);
-        const bool member = (sRef[slot] >> lane) & 1u;
-        const bool shared = sMul[slot * 32u + lane] > 1u;
+        const bool member = (S.ref[slot] >> lane) & 1u;
+        const bool shared = S.mul[slot * 32u + lane] > 1u;
         const uint32_t mS = __ballot_sync(kFull, member && shared), mE = __ballot_sync(kFull, member && !shared);
         const uint32_t sumS = __reduce_add_sync(kFull, (member && shared) ? acc[i] : 0u);
         const uint32_t sumE = __reduce_add_sync(kFull, (member && !shared) ? acc[i] : 0u);
         if (lane == 0) {
-          if (coinc && d.stats) atomicAdd(d.stats + 2, coinc);
+          if (coinc && (!MULTI || d.stats)) atomicAdd(d.stats + 2, coinc);
           if (mS) { atomicAdd(d.driveLog + tr * 4u + 0u, sumS); atomicAdd(d.driveLog + tr * 4u + 1u, (uint32_t)__popc(mS)); }
           if (mE) { atomicAdd(d.driveLog + tr * 4u + 2u, sumE); atomicAdd(d.driveLog + tr * 4u + 3u, (uint32_t)__popc(mE)); }
         }
       }
       if (lane == 0) {
-        if (d.hist) d.hist[(size_t)tr * ncol + cc] = bw;
-        if (bw != 0u && recur && d.stats) {
+        if (!MULTI || d.hist) d.hist[(size_t)tr * ncol + cc] = bw;
+        if (bw != 0u && recur && (!MULTI || d.stats)) {
           const uint32_t sb = 64u + tr * 8u;
           atomicAdd(d.stats + 0, 1u);
           atomicAdd(d.stats + 1, (uint32_t)__popc(bw));
@@ -167,10 +197,10 @@ struct PresentCta {
     };
 
     for (uint32_t t = 0; t < c.T; ++t) {
-      const uint32_t* sIn = (t & 1u) ? sSpk1 : sSpk0;
-      uint32_t* sOut = (t & 1u) ? sSpk0 : sSpk1;
-      const uint32_t* sActIn = (t & 1u) ? sAct1 : sAct0;
-      uint32_t* sActOut = (t & 1u) ? sAct0 : sAct1;
+      const uint32_t* sIn = (t & 1u) ? S.spk1 : S.spk0;
+      uint32_t* sOut = (t & 1u) ? S.spk0 : S.spk1;
+      const uint32_t* sActIn = (t & 1u) ? S.act1 : S.act0;
+      uint32_t* sActOut = (t & 1u) ? S.act0 : S.act1;
       const uint4* sIn4 = reinterpret_cast<const uint4*>(sIn);
       const uint32_t g = g0 + t, par = g & 1u, h3 = g % 3u;
       const bool clamp = t < c.clampSteps;
@@ -196,13 +226,13 @@ struct PresentCta {
         const bool on = (sActIn[cn[i] >> 5] >> (cn[i] & 31u)) & 1u;
         uint32_t active = __ballot_sync(kFull, on);
         const uint32_t n = (uint32_t)__popc(active);
-        nTiles += n;
+        if (MULTI) nTiles += n;
         uint32_t a = 0, b2 = 0;
         uint32_t slot0 = 0;
-        if (lane == 0 && n != 0u) slot0 = atomicAdd(sFlag + 3, n);
+        if (lane == 0 && n != 0u) slot0 = atomicAdd(S.flag + 3, n);
         slot0 = __shfl_sync(kFull, slot0, 0);
         const bool pooled = n != 0u && slot0 + n <= poolTiles;
-        uint64_t* mb = &sMbar[warp * CPW + (uint32_t)i];
+        uint64_t* mb = &S.mbar[warp * CPW + (uint32_t)i];
         if (pooled) {
           if (lane == 0) mbar_expect_tx(mb, n * 1024u);
           __syncwarp();
@@ -210,7 +240,7 @@ struct PresentCta {
             const uint32_t r = (uint32_t)__popc(active & ((1u << lane) - 1u));
             if (LEARN) fence_proxy_async_all();
             else fence_proxy_async_smem();
-            bulk_g2s(sPool + (size_t)(slot0 + r) * kTileU4, d.W3 + ((size_t)cc * kNslot + lane) * kTileU4, 1024u, mb);
+            bulk_g2s(S.pool + (size_t)(slot0 + r) * kTileU4, d.W3 + ((size_t)cc * kNslot + lane) * kTileU4, 1024u, mb);
           }
         }
         // a readout writes the previous step's records while this step's tiles are in flight
@@ -227,7 +257,7 @@ struct PresentCta {
             mbar_wait(mb, ph, c.waitNs > kDrainNs ? c.waitNs : kDrainNs);
           }
           mph ^= 1u << i;
-          const uint4* T = sPool + (size_t)slot0 * kTileU4 + lane;
+          const uint4* T = S.pool + (size_t)slot0 * kTileU4 + lane;
           for (uint32_t r = 0; active; ++r, T += kTileU4) {
             const uint32_t s = (uint32_t)(__ffs(active) - 1);
             active &= active - 1u;
@@ -267,7 +297,7 @@ struct PresentCta {
           }
         }
         if (c.facil != 0u && ((sIn[cc] >> lane) & 1u)) a += c.facil;
-        const uint32_t bi = c.useBias ? (sBias[(warp * CPW + (uint32_t)i) * 32u + lane] >> c.biasShift) : 0u;
+        const uint32_t bi = c.useBias ? (S.bias[(warp * CPW + (uint32_t)i) * 32u + lane] >> c.biasShift) : 0u;
         a = a > bi ? a - bi : 0u;
         acc[i] = a;
         bb[i] = b2;
@@ -290,7 +320,7 @@ struct PresentCta {
         __syncthreads();
         if (tid == 0) stamp[1] = globaltimer_ns();
       }
-      if (!grid_barrier(tm.bar, d.err, tm.nb + c.missing, g0 + t, c.waitNs, sFlag)) return false;
+      if (!grid_barrier(tm.bar, d.err, tm.nb + c.missing, g0 + t, c.waitNs, S.flag)) return false;
       if (stamp && tid == 0) stamp[2] = globaltimer_ns();
 
       // ---------------- phase B: column threshold (k_topk) and the full spike vector
@@ -298,25 +328,25 @@ struct PresentCta {
       // copies, in that order (three groups): warp 0 scans the histogram while the drives and
       // ballots keep arriving
       for (uint32_t i = tid; i < kHistWords / 4u; i += blockDim.x)
-        cp_async16(reinterpret_cast<uint4*>(sHist) + i, reinterpret_cast<const uint4*>(tm.hist + h3 * kHistWords) + i);
+        cp_async16(reinterpret_cast<uint4*>(S.hist) + i, reinterpret_cast<const uint4*>(tm.hist + h3 * kHistWords) + i);
       cp_async_commit();
       for (uint32_t i = tid; i < ncol / 4u; i += blockDim.x)
-        cp_async16(reinterpret_cast<uint4*>(sD) + i, reinterpret_cast<const uint4*>(d.xdrive + par * ncol) + i);
+        cp_async16(reinterpret_cast<uint4*>(S.drv) + i, reinterpret_cast<const uint4*>(d.xdrive + par * ncol) + i);
       cp_async_commit();
       for (uint32_t i = tid; i < ncol / 4u; i += blockDim.x)
-        cp_async16(reinterpret_cast<uint4*>(sB) + i, reinterpret_cast<const uint4*>(d.xball + par * ncol) + i);
+        cp_async16(reinterpret_cast<uint4*>(S.ball) + i, reinterpret_cast<const uint4*>(d.xball + par * ncol) + i);
       cp_async_commit();
-      if (tid == 0) { sFlag[2] = 0u; sFlag[3] = 0u; }  // every warp has claimed its pool slots
+      if (tid == 0) { S.flag[2] = 0u; S.flag[3] = 0u; }  // every warp has claimed its pool slots
       // histogram g+2 (last read in step g-1, before this barrier) is cleared for its next use
       if (tm.rank == 0 && g >= 1u)
         for (uint32_t i = tid; i < kHistWords; i += blockDim.x) __stcg(tm.hist + ((g + 2u) % 3u) * kHistWords + i, 0u);
       cp_async_wait<2>();  // the histogram
       __syncthreads();
-      const uint32_t theta = hist_theta<1>(sD, sHist, sCand, sFlag + 2, incols, ncol, c.targetCols, c.topkPar);
+      const uint32_t theta = hist_theta<1>(S.drv, S.hist, S.cand, S.flag + 2, incols, ncol, c.targetCols, c.topkPar);
       const uint32_t gate = max(theta, 1u);
       cp_async_wait<0>();
       __syncthreads();
-      emit_groups(sD, sB, sStim, sOut, sActOut, gate, clamp, incols, ngrp);
+      emit_groups(S.drv, S.ball, S.stim, sOut, sActOut, gate, clamp, incols, ngrp);
       __syncthreads();
       if (tm.rank == 0 && tid == 0) { d.theta[0] = theta; d.theta[1] = 0u; }
 
@@ -335,28 +365,28 @@ struct PresentCta {
         // k_bias, src/axon.mm:240-253
         if (recur) {
           const int dec = ((t % max(c.biasDownEvery, 1u)) == 0u) ? (int)c.biasDown : 0;
-          const int nb = (int)sBias[slot * 32u + lane] + (fired ? (int)c.biasUp : -dec);
-          sBias[slot * 32u + lane] = (uint32_t)max(0, nb);
+          const int nb = (int)S.bias[slot * 32u + lane] + (fired ? (int)c.biasUp : -dec);
+          S.bias[slot * 32u + lane] = (uint32_t)max(0, nb);
         }
         // k_learn, src/axon.mm:436-495: each voted branch of a learning column becomes a
         // task that any warp of the CTA runs, so a column's read-modify-writes overlap
         if (phase == 3u || b == 0u) continue;
         if (c.marginGate != 0u && !(vk[i] > vk1[i])) continue;
         const uint32_t vmask = __reduce_or_sync(kFull, fired ? bb[i] : 0u);
-        sBBL[slot * 32u + lane] = bb[i];
-        sLTP[slot * 32u + lane] = 0u;
-        sLTD[slot * 32u + lane] = 0u;
-        if (lane == 0) { sFiredL[slot] = b; sColL[slot] = cc; sMark[slot] = t + 1u; }
-        if ((vmask >> lane) & 1u) sTask[atomicAdd(sFlag + 1, 1u)] = (slot << 5) | lane;
+        S.bbl[slot * 32u + lane] = bb[i];
+        S.ltp[slot * 32u + lane] = 0u;
+        S.ltd[slot * 32u + lane] = 0u;
+        if (lane == 0) { S.firedL[slot] = b; S.colL[slot] = cc; S.mark[slot] = t + 1u; }
+        if ((vmask >> lane) & 1u) S.task[atomicAdd(S.flag + 1, 1u)] = (slot << 5) | lane;
       }
       if (LEARN) {
         __syncthreads();
-        const uint32_t ntask = sFlag[1];
-        nTasks += ntask;
+        const uint32_t ntask = S.flag[1];
+        if (MULTI) nTasks += ntask;
         for (uint32_t k = warp; k < ntask; k += wpb) {
-          const uint32_t tk = sTask[k], slot = tk >> 5, s = tk & 31u;
-          const uint32_t cc = sColL[slot];
-          const bool want = ((sFiredL[slot] >> lane) & 1u) && ((sBBL[slot * 32u + lane] >> s) & 1u);
+          const uint32_t tk = S.task[k], slot = tk >> 5, s = tk & 31u;
+          const uint32_t cc = S.colL[slot];
+          const bool want = ((S.firedL[slot] >> lane) & 1u) && ((S.bbl[slot * 32u + lane] >> s) & 1u);
           const uint32_t g = __ldg(d.conn + cc * kNslot + s);
           const size_t base = ((size_t)cc * kNslot + s) * kTileU4 + lane;
           uint4 p0[2], p1[2], p2[2], p3[2];
@@ -385,33 +415,33 @@ struct PresentCta {
             __stcg(d.W3 + base + 32 * j, p3[j]);
           }
           fence_proxy_async_all();  // the next step copies W3 tiles in bulk (async proxy)
-          if (nLTP) atomicAdd(sLTP + slot * 32u + lane, nLTP);
-          if (nLTD) atomicAdd(sLTD + slot * 32u + lane, nLTD);
+          if (nLTP) atomicAdd(S.ltp + slot * 32u + lane, nLTP);
+          if (nLTD) atomicAdd(S.ltd + slot * 32u + lane, nLTD);
         }
         __syncthreads();
         // plasticity counters per neuron and step, src/axon.mm:491-494
 #pragma unroll
         for (int i = 0; i < CPW; ++i) {
           const uint32_t slot = warp * CPW + (uint32_t)i;
-          if (col[i] >= ncol || sMark[slot] != t + 1u) continue;  // (helper warps own no column)
-          const uint32_t nLTP = sLTP[slot * 32u + lane], nLTD = sLTD[slot * 32u + lane];
+          if (col[i] >= ncol || S.mark[slot] != t + 1u) continue;  // (helper warps own no column)
+          const uint32_t nLTP = S.ltp[slot * 32u + lane], nLTD = S.ltd[slot * 32u + lane];
           const uint32_t sumP = __reduce_add_sync(kFull, nLTP), sumD = __reduce_add_sync(kFull, nLTD);
           const uint32_t kP = __popc(__ballot_sync(kFull, nLTP != 0u)), kD = __popc(__ballot_sync(kFull, nLTD != 0u));
-          if (lane == 0 && d.stats) {
+          if (lane == 0 && (!MULTI || d.stats)) {
             if (sumP) atomicAdd(d.stats + 8, sumP);
             if (sumD) atomicAdd(d.stats + 9, sumD);
             if (kP) atomicAdd(d.stats + 10, kP);
             if (kD) atomicAdd(d.stats + 11, kD);
           }
         }
-        if (tid == 0) sFlag[1] = 0u;
+        if (tid == 0) S.flag[1] = 0u;
       }
       __syncthreads();  // sOut / sActOut complete before the next step reads them
       if (stamp && tid == 0) stamp[4] = globaltimer_ns();
     }
 
     if (!LEARN) {  // the last step's records
-      const uint32_t* sLast = (c.T & 1u) ? sSpk1 : sSpk0;
+      const uint32_t* sLast = (c.T & 1u) ? S.spk1 : S.spk0;
 #pragma unroll
       for (int i = 0; i < CPW; ++i)
         if (col[i] < ncol) records(i, c.T - 1u, sLast[col[i]]);
@@ -420,10 +450,11 @@ struct PresentCta {
   }
 
   // final state of a presentation, as the reference's buffers hold it after present()
-  __device__ __forceinline__ void end(const NetDev& d, uint32_t T) {
+  __device__ __forceinline__ void end(const NetDev& d, const PresentTeam& tm, uint32_t T) {
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t* sLast = (T & 1u) ? sSpk1 : sSpk0;   // spk(T-1)
-    const uint32_t* sPrev = (T & 1u) ? sSpk0 : sSpk1;   // spk(T-2), zero when T == 1
+    const uint32_t* sLast = (T & 1u) ? S.spk1 : S.spk0;   // spk(T-1)
+    const uint32_t* sPrev = (T & 1u) ? S.spk0 : S.spk1;   // spk(T-2), zero when T == 1
     uint32_t* gLast = ((T - 1u) & 1u) ? d.spkA : d.spkB;
     uint32_t* gPrev = ((T - 1u) & 1u) ? d.spkB : d.spkA;
 #pragma unroll
@@ -437,11 +468,12 @@ struct PresentCta {
   }
 
   // the biases that learning changed
-  __device__ __forceinline__ void store_bias(const NetDev& d) {
+  __device__ __forceinline__ void store_bias(const NetDev& d, const PresentTeam& tm) {
+    const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < CPW; ++i)
-      if (col[i] < ncol) d.bias[col[i] * 32u + lane] = sBias[(warp * CPW + (uint32_t)i) * 32u + lane];
+      if (col[i] < ncol) d.bias[col[i] * 32u + lane] = S.bias[(warp * CPW + (uint32_t)i) * 32u + lane];
   }
 };
 
