@@ -27,9 +27,10 @@ constexpr int planes_threads(bool direct) { return direct ? 896 : 640; }
 constexpr uint32_t kPlanesDirectB = 160;            // most trajectories whose tiles are read through L2
 // up to this width every column with a drive is a candidate: storing their planes costs less than
 // recomputing gated columns after a threshold below the floor, which small networks meet often
-// (us of a 30-step call of 40 trajectories, bias off and on, floor / all: 256 columns 800 / 726 and
-// 1639 / 1076; 512: 806 / 671 and 922 / 869; 1,024: 740 / 772 and 1030 / 1042)
-constexpr uint32_t kPlanesAllCols = 512;
+// (us of a 30-step call, floor / all: 40 trajectories of whole cues 256 columns 800 / 726, 512: 806 /
+// 671, 1,024: 740 / 772; of three quarters of a cue 544: 725 / 575, 576: 710 / 601; 300
+// trajectories 544: 924 / 913, 576 with partial cues 1,093 / 993, 640: 913 / 1,055)
+constexpr uint32_t kPlanesAllCols = 576;
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 
 // A network and the team's words for it.

@@ -133,3 +133,13 @@ def test_small_networks(ncol, target, B):
     same(net, cues_of(net, pats, B, B), 12, 3, use_bias=1)
     same(net, cues_of(net, pats, B, B + 1), 12, 3, slab="floor_always")
     net.close()
+
+
+# the widths next to the line up to which every column with a drive is a candidate
+@pytest.mark.parametrize("ncol", [576, 608])
+@pytest.mark.parametrize("B", [5, 40, 200])
+def test_widths_about_the_candidate_line(ncol, B):
+    net, pats = trained(ncol=ncol, incols=72, target=9, k=24, nstim=12, epochs=2)
+    for bias in (0, 1):
+        same(net, cues_of(net, pats, B, B + bias), 12, 3, use_bias=bias)
+    net.close()
