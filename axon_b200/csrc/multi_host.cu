@@ -406,7 +406,11 @@ axon_status MultiRun::tune(Shape* best, std::vector<std::vector<uint32_t>>* best
   std::vector<uint64_t> cost(n_);
   for (uint32_t i = 0; i < n_; ++i) cost[i] = plans_[i].steps;
   const uint32_t slotCands[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 25, 32, 40, 50, 64, 74};
-  const int shapeCands[][2] = {{896, 0}, {1024, 4}, {896, 4}, {512, 8}};
+  // the first launch after the networks' initialisation is 8 to 17 % slower than a repeat, so that place
+  // goes to the shape that comes last in the others' order (one network of 352 to 4,096 columns: 1,024
+  // threads 20 to 70 % behind the best; with the pool form timed first it lost to 512 threads by that
+  // much, and the run took 4.7 instead of 4.1 ms at 352 columns, 21.6 instead of 17.7 at 4,096)
+  const int shapeCands[][2] = {{1024, 4}, {896, 4}, {512, 8}, {896, 0}};
   double bestT = 1e300;
   *tuneMs = 0.f;
   *tried = 0;
@@ -414,7 +418,9 @@ axon_status MultiRun::tune(Shape* best, std::vector<std::vector<uint32_t>>* best
     for (uint32_t S : slotCands) {
       if (S > n_ || S > grid) continue;
       const std::vector<uint32_t> ncta = split_ctas(grid, S);
-      if (sc[1] == 0 ? multi_pool_cpw(ncol_, incols_, *std::min_element(ncta.begin(), ncta.end())) == 0
+      // (with two columns per warp the pool form is level with the others and not worth its timing: 28.6 against
+      // 28.8 ms for two networks of 4,096 columns, 26.3 against 26.4 for two of 2,080)
+      if (sc[1] == 0 ? multi_pool_cpw(ncol_, incols_, *std::min_element(ncta.begin(), ncta.end())) != 1
                      : multi_smem_bytes(ncol_, incols_, max_cpw(ncta, sc[0]), sc[0]) > 227 * 1024)
         continue;
       // calibration: slot s runs network s for a few learning presentations
@@ -437,7 +443,10 @@ axon_status MultiRun::tune(Shape* best, std::vector<std::vector<uint32_t>>* best
       ++*tried;
       const double perStep = stepsPerSlot ? ms / (double)stepsPerSlot : 1e9;  // ms per step of one slot
       std::vector<std::vector<uint32_t>> queues;
-      const double span = assign(cost, ncta, queues) * perStep;
+      // the calibration's first presentations weigh learning more than the whole run does, where the pool form
+      // gains less: pool / 512 threads in it and in the run, one network of 352 columns 0.93 and 0.85, 1,024 in
+      // two slots 1.03 and 0.92, 2,080 0.95 and 0.90, 4,096 0.92 and 0.82
+      const double span = assign(cost, ncta, queues) * perStep * (sc[1] == 0 ? 0.92 : 1.0);
       if (span < bestT) {
         bestT = span;
         *best = sh;

@@ -45,3 +45,15 @@ def test_pool_equals_plain(ncol, incols, loads, slots, tiles):
                                      dict(biasdownevery=3, biasshift=2, ktest=8, facil=5)])
 def test_pool_rule_variants(variant):
     check(dict(ax.CONFIG_C, ncol=512, incols=64, target=24, **variant), [3, 4, 2], 2)
+
+
+# the tuner's choice takes no longer than the best of the shapes it chooses from (which are 15 % apart at
+# these widths; a tenth is allowed for the time of a launch)
+@pytest.mark.parametrize("ncol,load", [(352, 6), (2080, 8)])
+def test_tuner_finds_the_fastest_shape(ncol, load):
+    cfg = dict(ax.CONFIG_C, ncol=ncol, incols=ncol // 8 // 8 * 8, target=ncol // 64)
+    kw = dict(epochs=4, stimcols=ncol // 64, method="launch")
+    with ax.Network(cfg) as net:
+        forced = min(ax.multi_train([net], [1], [load], autotune=False, slots=1, threads=t, **kw)[1]["gpu_ms"]
+                     for t in (0, 512, 896, 1024) for _ in range(2))
+        assert ax.multi_train([net], [1], [load], **kw)[1]["gpu_ms"] <= 1.1 * forced
