@@ -16,11 +16,12 @@
 //            threshold (the target-th largest recurrent drive) and rebuilds the whole
 //            spike vector spk(t) in its own shared memory; no second barrier is needed.
 //   phase C  each warp finishes its own column: hist/stats/driveLog records, intrinsic
-//            bias (in a register for the whole launch) and bit-serial learning on W0..W3.
+//            bias and bit-serial learning on W0..W3.
 //
-// Per-neuron state that only its owner touches (bias, conn row, multiplicity) lives in
-// registers for the whole presentation; HBM traffic per step is the W3 tiles of
-// non-silent branches plus the learning read-modify-writes.
+// Per-neuron state that only its owner touches stays on the SM for the whole presentation
+// (the connection row in registers; bias and multiplicity in shared memory); HBM traffic
+// per step is the W3 tiles of non-silent branches plus the learning read-modify-writes.
+// The step loop is in present.cuh, which the multi-network launch shares.
 #include <cstdint>
 
 #include "axon_device.cuh"

@@ -14,8 +14,8 @@
 //            the lane's drive planes with ripple-carry logic operations: no population
 //            counts, no counters in shared memory, no atomics, no barrier between tasks.
 //            Column drives go to global memory; a column whose drive reaches the
-//            trajectory's floor (half its previous threshold) is a candidate: column, drive
-//            and drive planes are appended to the trajectory's list.
+//            trajectory's floor (mostly 5/8 of its threshold two steps back, cand_floor) is a
+//            candidate: a bit per column, and its drive planes, are kept for phase 2.
 //   barrier
 //   phase 2  a group of warps per trajectory: the column threshold from the candidates (from
 //            all drives, with the gated columns' planes recomputed, when fewer than `target`
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
   const bool sorted = !DIRECT || (nblk > 1u && ncols <= c.nl);
   const uint32_t ls = c.ls, tpw = 32u >> ls, ntb = sorted ? nblk << ls : (B + tpw - 1u) / tpw, ntask = ncols * ntb;
   const uint32_t part = lane & ((1u << ls) - 1u);
-  const uint32_t ntbInv = (uint32_t)((0x100000000ull + ntb - 1u) / ntb);  // k / ntb of a task (k < 2^16) by a product
+  const uint32_t ntbInv = (uint32_t)((0x100000000ull + ntb - 1u) / ntb);  // k / ntb of a task by a product (exact while k * ntb < 2^32: at most 8,192 columns x 16 tasks)
 
   if (tid == 0) {
     for (uint32_t i = 0; i < kMaxNS + kMaxNL; ++i) mbar_init(&sBarT[i], 1);

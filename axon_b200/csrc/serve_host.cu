@@ -2,12 +2,15 @@
 //
 // The reference answers one readout at a time (present() with learn = 0,
 // src/axon.mm:815-888). The server accepts recall requests (network, cue columns, clamped
-// and free steps) at any time and runs them on an internal thread, tick by tick: at every
-// tick it admits requests that have arrived into free trajectory slots (the slot count is
-// set by the device-memory budget given at creation), advances every admitted trajectory
-// by one step in one batched pass (serve.cu), and retires the trajectories whose last step
-// ran, with their final spikes. A request's result does not depend on what else is in
-// flight: every trajectory reads only its own slot and the network's read-only weights.
+// and free steps) at any time and runs them on an internal thread, launch by launch: before
+// each it admits requests that have arrived into free trajectory slots (the slot count is
+// set by the device-memory budget given at creation), then it advances every admitted
+// trajectory, and retires those whose last step ran, with their final spikes. On the bit
+// planes (serve_planes.cu) a launch runs up to kServeSteps steps, fewer when a trajectory ends
+// or a request is known to arrive before that: a request that was not announced waits up to
+// so many steps to be admitted. Outside the planes' range (serve.cu, serve_batched.cu) it is
+// one step. A request's result does not depend on what else is in flight: every trajectory
+// reads only its own slot and the network's read-only weights.
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>

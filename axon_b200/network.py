@@ -123,10 +123,11 @@ class Network:
 
         contraction: "popc" (CUDA cores) or "tensor" (binary MMA) computes the batched
         method's AND-popcounts; the results are the same.
-        slab: which per-neuron drives the batched method stores for the k-of-32 of gated
-        columns: "floor" (columns at or above the trajectory's histogram floor, all of them
-        at the step after the clamp), "floor_always" or "full"; gated columns without a
-        stored drive are recomputed, and the results are the same.
+        slab: whose per-neuron drives the batched method keeps for the k-of-32 of gated
+        columns: "floor" (columns at or above a floor from the trajectory's earlier
+        thresholds), "floor_always" (without the floor's rule for the step after the clamp)
+        or "full" (every column); gated columns without a kept drive are recomputed, and the
+        results are the same.
 
         Returns {"final": (B, ncol), "hist": (B, T, ncol) | None, "stats": (B, 1024) | None,
         "drive_log": (B, 256) | None, "gpu_ms": float}. final_out, a C-contiguous uint32

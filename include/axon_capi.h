@@ -170,8 +170,9 @@ uint32_t axon_noisy_cue_seed(uint32_t q, uint32_t pct, uint32_t draw);
  * spikes of every step, stats B*1024 counters of k_emit (word 2, the branch-coincidence
  * count, is produced by the plain method only), drive_log B*256 added to like the
  * reference's driveLog buffer for the members marked in ref_ball (B*ncol, NULL = none;
- * the shared/exclusive split uses the network's MULT buffer). gpu_ms receives the
- * device time of the launches. The network's per-present buffers are left undefined. */
+ * the shared/exclusive split uses the network's MULT buffer; the batched method ignores
+ * ref_ball when drive_log is NULL). gpu_ms receives the device time of the launches. The
+ * network's per-present buffers are left undefined. */
 typedef enum axon_recall_method { AXON_RECALL_BATCHED = 0, AXON_RECALL_PLAIN = 1 } axon_recall_method;
 
 typedef struct axon_recall_args {
@@ -313,10 +314,14 @@ axon_status axon_multi_train(axon_net* const* nets, uint32_t n, const uint32_t* 
  * The reference runs one readout at a time: present() with learn = 0 (src/axon.mm:815-888),
  * the clamp built from a pattern's kept columns (src/axon.mm:800-804). A server answers
  * such readouts as requests against device-resident trained networks, with continuous
- * batching: an internal thread advances, tick by tick, every admitted trajectory by one
- * step in one batched pass (trajectories of one network share each weight-tile load),
- * admits requests that have arrived into slots as they free up (the slot count follows
- * from mem_bytes, the device memory the server may use), and retires finished ones. A
+ * batching: an internal thread advances every admitted trajectory together (trajectories
+ * of one network share each weight-tile load), admits requests that have arrived into slots
+ * as they free up (the slot count follows from mem_bytes, the device memory the server may
+ * use), and retires finished ones. One launch runs up to eight steps, fewer when a
+ * trajectory ends or a submitted request's arrive_s falls before that; a request that was
+ * not announced by its arrive_s waits for the running launch (with facilitation or boosts
+ * of 256 and more a launch is one step). Where the layout that this needs does not fit the
+ * device's memory the server takes the older one-step form, with the same results. A
  * request's final spikes are the same as those of axon_recall for the same network, cue
  * and steps, whatever else is in flight. The networks must share one axon_cfg and device
  * and must not be changed (present, write, init) while the server exists.
@@ -336,11 +341,11 @@ typedef struct axon_serve_counters {
   uint32_t slots;      /* trajectory slots the memory budget allows */
   uint32_t in_flight;  /* slots in use now */
   uint64_t queued;     /* submitted, not yet admitted */
-  uint64_t ticks;      /* batched steps run */
+  uint64_t ticks;      /* batched steps run (a launch of several counts as many) */
   uint64_t completed;  /* requests finished */
-  uint64_t max_batch;  /* most trajectories advanced in one tick */
+  uint64_t max_batch;  /* most trajectories advanced in one launch */
   double mean_batch;   /* trajectories per tick, mean */
-  double busy_s;       /* time spent in ticks */
+  double busy_s;       /* time spent in launches, their tables and results */
   double drive_s;      /* device time of the drive kernel, summed over ticks (of the whole step when one kernel runs it) */
   double emit_s;       /* device time of the threshold/emit kernel, summed over ticks */
   uint64_t slot_bytes; /* device memory one trajectory slot takes */
