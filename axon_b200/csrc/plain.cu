@@ -34,7 +34,7 @@ namespace axon {
 
 template <int CPW, bool LEARN>
 __global__ void __launch_bounds__(kPresentMaxWarps * 32, 1) k_present(NetDev d, PresentCfg c) {
-  const PresentTeam tm{blockIdx.x, gridDim.x, c.ownWarps, present_smem_layout(c.ncol, c.incols, CPW).poolTiles, d.bar,
+  const PresentTeam tm{blockIdx.x, gridDim.x, LEARN ? c.ownWarps : blockDim.x >> 5, present_smem_layout(c.ncol, c.incols, CPW).poolTiles, d.bar,
                        d.bar + 64};
   PresentCta<CPW, false> w;
   w.init(c.ncol, c.incols, tm);

@@ -138,10 +138,11 @@ struct PresentCta {
   // carry none of the learning code's register pressure. Returns false when a grid wait gave up.
   template <bool LEARN>
   __device__ __forceinline__ bool steps(const NetDev& d, const PresentCfg& c, const PresentTeam& tm, uint32_t g0) {
-    // a readout takes the sizes from the kernel's parameters, and the shared-memory map from them, instead of
-    // holding them for the launch: a step of 2,080 columns takes 6.35 us (drive 2.21, spikes 1.82) against 6.47
-    // (2.25, 1.88). Learning is the other way round (a 10-step presentation of 4,096 columns 202 against 189 us)
-    const uint32_t ncol = MULTI || LEARN ? this->ncol : c.ncol, incols = MULTI || LEARN ? this->incols : c.incols;
+    // the sizes, and the shared-memory map from them, come from the kernel's parameters instead of being held
+    // for the launch: a readout step of 2,080 columns takes 6.35 us (drive 2.21, spikes 1.82) against 6.47
+    // (2.25, 1.88), a 10-step learning call of 6,144 columns 252 against 260 us. Learning with one column per
+    // warp is the other way round (4,096 columns: 202 against 189 us)
+    const uint32_t ncol = MULTI || (LEARN && CPW == 1) ? this->ncol : c.ncol, incols = MULTI || (LEARN && CPW == 1) ? this->incols : c.incols;
     const PresentMap S = present_map(ncol, incols, tm.own * CPW, CPW);
     const uint32_t ngrp = ncol / 8u, poolTiles = tm.poolTiles;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, wpb = blockDim.x >> 5;
