@@ -88,7 +88,8 @@ struct PlanesDev {
 struct PlanesCfg {
   uint32_t ncol, incols, B, T, clampSteps, k, dthr, mode, targetCols, topkPar;
   uint32_t bst;          // dendritic bonus per branch at or above dthr: boost (mode 1), 0 (mode 0)
-  uint32_t slabFull;     // 1: every column with a positive drive is a candidate
+  uint32_t allCand;      // 1: every column with a positive drive is a candidate
+  uint32_t storeAll;     // 1: every column with a positive drive keeps its planes, candidate or not
   uint32_t slabAlways;   // 1: the first step after the clamp takes no floor of its own
   uint32_t ns, nl, ng;   // tile slots, list slots (0 when direct), phase-2 groups
   uint32_t nsl, nll;     // log2 of ns and nl

@@ -429,7 +429,7 @@ __device__ __forceinline__ uint32_t plane_kwta(const uint32_t (&D)[kPlanes], uin
 // phase 2 selects from all drives.
 __device__ __forceinline__ uint32_t cand_floor(const uint32_t* thPrev, uint32_t stride, uint32_t b, uint32_t t,
                                                uint32_t clampSteps, const PlanesCfg& c) {
-  if (c.slabFull) return 1u;
+  if (c.allCand) return 1u;
   if (t <= 1u) return t ? 0xFFFFFFFFu : 1u;
   const bool drop = t == clampSteps + 1u && !c.slabAlways;
   const bool next = t == clampSteps + 2u, one = drop || next || t == 2u;
@@ -852,10 +852,9 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
             if (sh) { atomicAdd(dl + 0, plane_sum(A, sh)); atomicAdd(dl + 1, (uint32_t)__popc(sh)); }
             if (ex) { atomicAdd(dl + 2, plane_sum(A, ex)); atomicAdd(dl + 3, (uint32_t)__popc(ex)); }
           }
-          if (s >= sFloor[b]) {
-            atomicOr(d.candB + (size_t)sl * (ncol / 32u) + (col >> 5), 1u << (col & 31u));
-            store_planes(d.candP + ((size_t)sl * ncol + col) * 4u, A);
-          }
+          const bool cand = s >= sFloor[b];
+          if (cand) atomicOr(d.candB + (size_t)sl * (ncol / 32u) + (col >> 5), 1u << (col & 31u));
+          if (cand || (!SERVE && c.storeAll != 0u && s != 0u)) store_planes(d.candP + ((size_t)sl * ncol + col) * 4u, A);
         }
         if (last) {
           __syncwarp();
@@ -926,7 +925,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
       grp.sync();
       uint32_t n = sR[60], theta = 1u;
       // too many candidates for the group's memory, or a threshold below the floor: the select
-      // runs on all drives, and the gated columns' planes are recomputed
+      // runs on all drives, and in the second case the gated columns' planes are recomputed
       bool redo = n > nV;
       uint4* candb = d.candP + (size_t)sl * ncol * 4u;
       uint32_t* candW = reinterpret_cast<uint32_t*>(candb);  // 16 words per column
@@ -1012,7 +1011,7 @@ __global__ void __launch_bounds__(planes_threads(DIRECT), 1) k_recall_planes(con
       // more gated columns than the list holds: all entries are walked and their spikes wait in global memory
       const bool over = npend > kPlanesList;
       const uint32_t walk = over ? n : npend;
-      if (redo)
+      if (redo && gate < fl && c.storeAll == 0u)  // (at or above the floor they were stored)
         for (uint32_t i = grp.t; i < walk; i += grp.nt) {
           const uint32_t e = over ? i : sList[i];  // = the column
           if (over && !gated(val(e))) continue;

@@ -87,7 +87,8 @@ axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axo
   c.ncol = ncol; c.incols = cfg.incols; c.T = a.T; c.clampSteps = a.clamp_steps;
   c.k = pc.k; c.dthr = pc.dthr; c.mode = pc.mode; c.targetCols = pc.targetCols; c.topkPar = pc.topkPar;
   c.bst = cfg.mode == 1 ? cfg.boost : 0u;
-  c.slabFull = a.slab == AXON_SLAB_FULL || (a.slab == AXON_SLAB_FLOOR && ncol <= kPlanesAllCols) ? 1u : 0u;
+  c.allCand = a.slab != AXON_SLAB_FLOOR_ALWAYS && ncol <= kPlanesAllCols ? 1u : 0u;
+  c.storeAll = a.slab == AXON_SLAB_FULL ? 1u : 0u;
   c.slabAlways = a.slab == AXON_SLAB_FLOOR_ALWAYS ? 1u : 0u;
   c.waitNs = wait_ns;
   const size_t nblk = (Bc + 31u) / 32u, bnc = (size_t)Bc * ncol;

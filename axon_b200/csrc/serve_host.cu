@@ -293,7 +293,7 @@ axon_status axon_server::start_planes(uint64_t memBytes) {
   dev.err = pdev.err;
   pcfg.ncol = ncol; pcfg.incols = incols; pcfg.k = cfg.k; pcfg.dthr = cfg.dthr; pcfg.mode = cfg.mode;
   pcfg.targetCols = cfg.targetCols; pcfg.topkPar = cfg.topkPar; pcfg.bst = cfg.bst; pcfg.waitNs = nets[0]->wait_ns;
-  pcfg.slabFull = ncol <= kPlanesAllCols ? 1u : 0u;
+  pcfg.allCand = ncol <= kPlanesAllCols ? 1u : 0u;
   CKS(planes_serve_prepare(pcfg));
   CKS(cudaStreamSynchronize(stream));
   for (uint32_t s = nslots; s-- > 0;) freeSlots.push_back(s);

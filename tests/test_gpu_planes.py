@@ -143,3 +143,15 @@ def test_widths_about_the_candidate_line(ncol, B):
     for bias in (0, 1):
         same(net, cues_of(net, pats, B, B + bias), 12, 3, use_bias=bias)
     net.close()
+
+
+# more candidates than a group keeps in shared memory (1,024), whose planes are stored: with biases every column
+# that passes a low floor; and every column's planes kept beside the candidates
+@pytest.mark.parametrize("ncol", [1056, 2080])
+def test_more_candidates_than_a_group_holds(ncol):
+    net, pats = trained(ncol=ncol, incols=128, target=32, k=24, epochs=2)
+    for B in (20, 170):
+        for slab in ("floor", "floor_always", "full"):
+            for bias in (0, 1):
+                same(net, cues_of(net, pats, B, B), 12, 3, slab=slab, use_bias=bias)
+    net.close()
