@@ -24,6 +24,10 @@ PresentCfg make_present_cfg(const axon_cfg& c, uint32_t T, uint32_t clampSteps, 
 // Whether the bit-plane readout takes this configuration: per-neuron drives below 2^14 (drive
 // << 13 | column fits one word), no facilitation.
 bool planes_config(const axon_cfg& cfg);
+// Whether it is also the faster form for a batch of B trajectories (bias: with biases, logged:
+// with a member-drive log), or for a server of such networks.
+bool planes_pay(const axon_cfg& cfg, uint32_t B, bool bias, bool logged);
+bool planes_pay_serving(const axon_cfg& cfg);
 // Co-resident launch shape of k_present for a network of ncol columns on a GPU with `sms`
 // SMs: one column per warp when the grid fits in one wave, else two.
 axon_status pick_present_shape(uint32_t ncol, uint32_t incols, int sms, LaunchShape* out);

@@ -77,6 +77,70 @@ bool axon::planes_config(const axon_cfg& cfg) {
   return cfg.facil == 0u && maxAcc < (1ull << kPlanes) && cfg.ncol <= 8192u;
 }
 
+namespace {
+// How a configuration loads the bit planes. A spike word of k neurons costs the sum of the masks of
+// the k it holds or of the 32 - k it leaves out, whichever are fewer: up to 8 left out take the main
+// loop, others a loop over the masks. And every winning column beyond one per group of eight
+// is a word more per branch, and a gated column more.
+struct PlanesLoad {
+  bool few, mid, hard;           // masks: at most 8 held; 9 to 12; 13 to 16
+  bool busy, dense, veryDense;   // target columns: above 1/18, 1/6, 1/3 of the recurrent ones
+};
+PlanesLoad planes_load(const axon_cfg& c) {
+  const uint32_t k = c.ktest ? c.ktest : c.k, rec = c.ncol - c.incols;
+  PlanesLoad l{};
+  l.few = k <= 8u;
+  l.hard = k >= 13u && k <= 19u;
+  l.mid = !l.few && !l.hard && k < 24u;
+  const uint64_t t = c.target == 0u ? rec : c.target;  // no target: every driven column spikes
+  l.busy = 18u * t > rec;
+  l.dense = 6u * t > rec;
+  l.veryDense = 3u * t > rec;
+  return l;
+}
+}  // namespace
+
+// The lines are where the former kernel (batch.cu) was measured faster, over 512, 1,312 and 4,096
+// columns, 1 to 512 trajectories and 30 steps. Its time over the bit planes' (below 1: it is faster):
+//                               at 1 / 13 / 40 / 100 / 170 / 300 trajectories of 4,096 columns, and of 512
+//   k 24, 64 of 4,096 columns   4.3 3.5 2.3 1.7 1.2 1.3                    1.3 1.6 1.5 1.4 1.4 1.4
+//   k 16                        2.9 2.1 1.0 0.8 0.7 0.8                    0.9 1.0 0.8 0.7 0.9 0.9
+//   k 10                        3.5 2.4 1.3 1.0 0.9 1.0                    1.1 1.1 0.9 0.7 0.8 0.9
+//   k 4                         2.7 2.0 1.2 1.0 1.0 1.0                    1.2 1.2 0.9 0.8 0.9 1.1
+//   1/12 of the columns         2.1 1.1 0.8 1.0 1.2 1.4                    1.2 1.0 0.8 0.9 1.2 1.4
+//   1/4                         1.3 0.9 0.9 1.1 1.2 1.3                    1.1 0.9 0.9 0.9 1.2 1.5
+//   boost 200                   2.8 2.3 1.7 1.2 1.0 1.0                    1.3 1.3 1.2 1.0 1.0 0.9
+//   biases, k 16                2.3 1.5 0.8 0.8 0.9 0.9                    0.8 0.7 0.6 0.5 0.7 0.9
+//   biases, 1/12                2.2 1.4 1.1 1.3 1.4 1.5                    1.3 1.1 1.0 1.1 1.3 1.6
+bool axon::planes_pay(const axon_cfg& c, uint32_t B, bool bias, bool logged) {
+  const PlanesLoad l = planes_load(c);
+  const bool lean = !bias && !logged;  // the former kernel's fast write-back
+  const bool small = c.ncol <= kPlanesAllCols, some = B <= 20u, many = B > 128u;
+  // candidates fit a group's memory but often miss the threshold, and half the columns are recomputed
+  // (target half of 1,312 columns: 0.3 to 0.6 up to 40 trajectories, with a log 0.2 to 0.7 for all)
+  if (l.veryDense && !small && c.ncol < 2048u) return lean && many;
+  if (l.dense && !many && (!bias || (small && !some))) return false;
+  if (l.busy && !l.dense && lean && !some && !many) return false;
+  if (l.hard) {
+    if (bias) return c.ncol >= 2048u && some;
+    if (logged) return c.ncol >= 2048u || many || (!small && some);
+    return !small && B <= (c.ncol >= 2048u ? 48u : 20u);
+  }
+  if (l.few && small && lean) return some || B > 256u;
+  if (l.mid && lean) return some || (!small && (B <= 96u || B > 256u));
+  if (l.mid && bias && small) return some || many;
+  if (lean && many && ((c.mode == 2u && c.dthr > 1u) || (c.mode == 1u && c.boost > 64u))) return false;
+  return true;
+}
+
+// Bursts of 8 / 60 / 300 requests, former kernels' time over the bit planes': k 16 1.1 / 0.9 / 0.8 at 4,096
+// columns, half the columns 0.6 / 1.0 / 1.2 there and 0.3 / 0.4 / 0.5 at 1,312, all 0.9 / 1.0 / 1.3; k 10 1.4 /
+// 1.2 / 1.0, a quarter of the columns 0.9 / 1.1 / 1.3.
+bool axon::planes_pay_serving(const axon_cfg& c) {
+  const PlanesLoad l = planes_load(c);
+  return !l.hard && !l.veryDense;
+}
+
 axon_status axon_net::recall_planes(const uint32_t* dCues, uint32_t B, const axon_recall_args& a, const uint32_t* dRef,
                                     uint32_t* dFinal, uint32_t* dHist, uint32_t* dStats, uint32_t* dLog) {
   axon_status st = ensure_w3p();
@@ -241,6 +305,8 @@ axon_status axon_net::recall(const uint32_t* cues, uint32_t B, const axon_recall
 
   float gpu_ms = 0.f;
   bool planes = a.method == AXON_RECALL_BATCHED && a.contraction == AXON_CONTRACT_POPC && planes_config(cfg);
+  if (planes && !planes_pay(cfg, B, a.use_bias != 0u, dRef != nullptr))
+    planes = ensure_w3b() == AXON_ENOMEM;  // the former kernel's layout does not fit beside what is there
   if (planes) {
     const axon_status st = recall_planes(dCues, B, a, dRef, dFinal, dHist, dStats, dLog);
     if (st != AXON_OK && st != AXON_ENOMEM) return st;

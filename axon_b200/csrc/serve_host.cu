@@ -168,7 +168,7 @@ axon_status axon_server::start(axon_net* const* ns, uint32_t n, uint64_t memByte
   capB = packed ? kServeMaxB : kServeMaxB32;
   CKS(cudaSetDevice(device));
   // the bit-plane form where it applies and its layout fits the device's memory
-  planes = planes_config(n0->cfg) && n <= (uint32_t)sms;
+  planes = planes_config(n0->cfg) && planes_pay_serving(n0->cfg) && n <= (uint32_t)sms;
   for (uint32_t i = 0; planes && i < n; ++i) {
     planes = nets[i]->ensure_w3p() == AXON_OK;
     if (planes) CKS(cudaStreamSynchronize(nets[i]->stream));

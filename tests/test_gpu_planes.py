@@ -155,3 +155,43 @@ def test_more_candidates_than_a_group_holds(ncol):
             for bias in (0, 1):
                 same(net, cues_of(net, pats, B, B), 12, 3, slab=slab, use_bias=bias)
     net.close()
+
+
+# both sides of the lines between this kernel and the former one: winners per column, share of winning columns,
+# number of trajectories, width, biases and logs
+@pytest.mark.parametrize("kw", [dict(k=6), dict(k=10), dict(k=16), dict(k=22), dict(target=40), dict(target=150), dict(target=0),
+                                dict(mode=2, dthr=2), dict(boost=200)])
+@pytest.mark.parametrize("ncol", [512, 608, 2080])
+def test_lines_between_the_kernels(kw, ncol):
+    net, pats = trained(**dict(dict(ncol=ncol, incols=64, target=8, k=24, epochs=1), **kw))
+    rng = np.random.default_rng(ncol)
+    for B in (20, 21, 48, 49, 97, 129):
+        cues = cues_of(net, pats, B, B)
+        same(net, cues, 9, 3)
+        same(net, cues, 9, 3, use_bias=1)
+        same(net, cues, 9, 3, ref_ball=rng.integers(0, 1 << 32, cues.shape, dtype=np.uint64).astype(np.uint32))
+    with ax.Server([net], 64 << 20) as srv:
+        for tag in range(30):
+            srv.submit(0, np.sort(pats[tag % 6][: 4 + tag % 9]).astype(np.uint32), 3, 4 + tag % 3, tag)
+        srv.wait_idle(60)
+        for res, spikes in srv.poll(30):
+            t = res["tag"]
+            cue = ax.clamp_words(np.sort(pats[t % 6][: 4 + t % 9]), ncol)[None]
+            assert np.array_equal(spikes, net.recall(cue, 7 + t % 3, 3, method="plain")["final"][0]), t
+    net.close()
+
+
+# the same above the width up to which every column is a candidate: a threshold below the floor in the step of the
+# move recomputes columns from the old lanes' activity words
+@pytest.mark.parametrize("target", [24, 150])
+def test_server_moves_lanes_of_wider_networks(target):
+    test_server_moves_lanes(dict(ncol=608, incols=72, target=target), 1)
+
+
+# more gated columns than the list holds, over the forms that keep this kernel for them
+@pytest.mark.parametrize("ncol,target,B,bias", [(2208, 1900, 130, 0), (2208, 600, 20, 1), (512, 440, 130, 0), (512, 440, 9, 1)])
+def test_more_gated_columns_than_the_list_holds(ncol, target, B, bias):
+    net, pats = trained(ncol=ncol, incols=64, target=target, k=24, epochs=1)
+    for slab in ("floor", "floor_always", "full"):
+        same(net, cues_of(net, pats, B, B), 9, 3, slab=slab, use_bias=bias)
+    net.close()
