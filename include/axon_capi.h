@@ -190,9 +190,10 @@ typedef struct axon_recall_args {
                            the results are the same */
   uint32_t slab;        /* batched method: whose per-neuron drives the kernel keeps for the k-of-32 of the columns
                            that pass the gate; the results are the same. AXON_SLAB_FLOOR (0): those of columns
-                           whose drive reaches a floor taken from the trajectory's earlier thresholds (with
-                           facilitation, drives of 2^14 and more, or the tensor contraction, half the previous one
-                           and every column at the step after the clamp); AXON_SLAB_FLOOR_ALWAYS (1): the same
+                           whose drive reaches a floor taken from the trajectory's earlier thresholds (where the
+                           form without bit planes runs, half the previous one and every column at the step after
+                           the clamp: facilitation, drives of 2^14 and more, the tensor contraction, and
+                           configurations that it is faster for); AXON_SLAB_FLOOR_ALWAYS (1): the same
                            without a rule of its own for the step after the clamp; AXON_SLAB_FULL (2): every one.
                            A gated column without a kept drive has it recomputed */
   uint32_t reserved[1]; /* zero */
@@ -319,8 +320,9 @@ axon_status axon_multi_train(axon_net* const* nets, uint32_t n, const uint32_t* 
  * as they free up (the slot count follows from mem_bytes, the device memory the server may
  * use), and retires finished ones. One launch runs up to eight steps, fewer when a
  * trajectory ends or a submitted request's arrive_s falls before that; a request that was
- * not announced by its arrive_s waits for the running launch (with facilitation or boosts
- * of 256 and more a launch is one step). Where the layout that this needs does not fit the
+ * not announced by its arrive_s waits for the running launch (with facilitation, boosts of
+ * 256 and more, 13 to 19 winners per column or more than a third of the columns winning a
+ * launch is one step). Where the layout that this needs does not fit the
  * device's memory the server takes the older one-step form, with the same results. A
  * request's final spikes are the same as those of axon_recall for the same network, cue
  * and steps, whatever else is in flight. The networks must share one axon_cfg and device
