@@ -637,8 +637,8 @@ def main() -> None:
                        "faster": min(per, key=per.get),
                        "note": "tensor = mma.sync m16n8k256 b1 and.popc, 8 entries x 32 rows per chunk; popc = __popc "
                                "on the CUDA cores"}
-        # A/B of the drive slab: every per-neuron drive stored (full) against only those at or
-        # above each trajectory's histogram floor (the default)
+        # A/B of the kept drives: every column's (full) against those at or above each trajectory's
+        # floor (the default)
         rf = net.recall(cues, T_RECALL, CLAMP_RECALL, hist=True, contraction=ctr, slab="full")
         full_exact = bool(np.array_equal(rf["hist"], ref["hist"]))
         for _ in range(args.warmup):
@@ -646,8 +646,8 @@ def main() -> None:
                               contraction=ctr, slab="full")
         tf = time_device(net, d_cues, B, T_RECALL, CLAMP_RECALL, d_fw, flush, max(5, args.steps // 2), ctr, "full")
         slab = {"floor_ms_per_step": ms, "full_ms_per_step": rep.max(float(np.mean(tf))), "full_bit_exact": full_exact,
-                "note": "floor = per-neuron drives stored for columns at or above the trajectory's histogram floor "
-                        "(all at the step after the clamp; gated columns without one recomputed); full = all stored"}
+                "note": "floor = per-neuron drives kept for columns at or above a floor from the trajectory's earlier "
+                        "thresholds (gated columns without them recomputed); full = kept for all"}
 
     # plain GPU path on the same 300 trajectories (one persistent launch per trajectory)
     plain = None
