@@ -635,8 +635,8 @@ def main() -> None:
         contraction = {"popc_ms_per_step": per["popc"], "tensor_ms_per_step": per["tensor"],
                        "timed_as_value": ctr, f"{other}_bit_exact": other_exact,
                        "faster": min(per, key=per.get),
-                       "note": "tensor = mma.sync m16n8k256 b1 and.popc, 8 entries x 32 rows per chunk; popc = __popc "
-                               "on the CUDA cores"}
+                       "note": "tensor = mma.sync m16n8k256 b1 and.popc, 8 entries x 32 rows per chunk; popc = logic "
+                               "operations on bit planes, on the CUDA cores"}
         # A/B of the kept drives: every column's (full) against those at or above each trajectory's
         # floor (the default)
         rf = net.recall(cues, T_RECALL, CLAMP_RECALL, hist=True, contraction=ctr, slab="full")
